@@ -13,14 +13,16 @@
 //     tests one node per step with all 32 lanes);
 //   - a node is accepted without a vote when the distance from its centre of
 //     mass to the group's bounding box already satisfies the criterion with a
-//     2^-16 relative margin (which dominates every rounding difference), and
-//     opened without a vote when a representative body (the group's body
-//     nearest the box corner on the node's side) already fails it;
-//     only the rest take the exact group vote (same FP32 operations and
-//     order as the reference, so the decision is bit-identical), two nodes
-//     per pass with packed FP32x2 arithmetic on a compacted copy of them,
-//     each lane collecting its body's verdicts in a bit mask that one warp OR
-//     combines;
+//     2^-16 relative margin (which dominates every rounding difference): 78%
+//     of the nodes tested (1M disk);
+//   - the others wait in a buffer until 32 are there.  Then each lane takes
+//     one and opens it when a representative body (the group's body nearest
+//     the box corner on the node's side) already fails the test; what is left
+//     (9% of the nodes) waits in a second buffer for the exact group vote,
+//     again 32 nodes at a time, one per lane, each lane running over the
+//     group's bodies two at a time with packed FP32x2 arithmetic (same FP32
+//     operations and order as the reference, so the decision is bit-identical);
+//     opened nodes push their children;
 //   - accepted nodes' (centre of mass, mass) are appended to a per-warp list
 //     in shared memory and evaluated in bulk, two list entries per
 //     instruction with sm_100's packed FP32x2 arithmetic: per pair of
@@ -31,6 +33,17 @@
 //   - sums are compensated per block of list entries (Kahan on the block
 //     partials) when requested;
 //   - warps fetch groups from an atomic cursor (dynamic load balance).
+// What bounds it: instruction dispatch.  A packed FP32x2 instruction takes two
+// dispatch cycles of a sub-partition, three when its three operands are
+// distinct registers; counted so, dispatch is 94% busy (262K learned walk: 28.6K
+// instructions and 13.3K packed second cycles per group in 47.8K cycles), 68% of it the
+// evaluation at 15-16 cycles per 32 interactions (14 without register-port
+// conflicts).  Everything that shortens the traversal's instruction stream
+// therefore shows: waiting for full batches of 32 before the rarer, dearer
+// tests (instead of running them, mostly empty, in every round) and explicit
+// shared addresses took the 1M disk's walk from 1873 to 1647 us (learned, RMS
+// 1e-3) and from 1587 to 1423 us (theta 0.5), and the 4M merger's step from
+// 9.18 to 8.18 ms.
 // Leaves never open, as in the reference (count <= 1 or no children).
 // Extensions (template switches, off for the reference's semantics): the
 // relative opening criterion with per-group budgets (the learned criterion),
@@ -56,7 +69,7 @@ constexpr int kThreads = kWarpsPerBlock * 32;
 constexpr int kStackSmemDefault = BH_WALK_STACK_SMEM;
 constexpr int kListCap = BH_WALK_LIST_CAP;      // interaction-list entries per warp (a multiple of 64)
 #ifndef BH_WALK_MIN_BLOCKS_PLAIN
-#define BH_WALK_MIN_BLOCKS_PLAIN 7
+#define BH_WALK_MIN_BLOCKS_PLAIN 6
 #endif
 #ifndef BH_WALK_MIN_BLOCKS_RELATIVE
 #define BH_WALK_MIN_BLOCKS_RELATIVE 6
@@ -66,11 +79,11 @@ constexpr int kListCap = BH_WALK_LIST_CAP;      // interaction-list entries per 
 #endif
 // Resident blocks per SM the register allocation must allow (64K registers /
 // (128 threads x blocks)): fewer blocks, more registers per thread.  Measured
-// on the 1M disk, the walk is faster with registers than with warps: 7 blocks
-// (72 registers) for the fixed-theta walks, 6 (80) with the relative test.
-// With the 256-entry list and the default 768-entry stack, shared memory
-// (38 KB per block) binds first: 5 blocks per SM, which measured faster than
-// 6 blocks with a 192-entry list.
+// on the 1M disk, the walk is faster with registers than with warps: 6 blocks
+// (80 registers), which is also what shared memory allows with the 256-entry
+// list and the default 768-entry stack (38 KB per block): 1652 us learned, 1432
+// plain; 7 blocks (72 registers, 512-entry stack) 1751 and 1465, 8 blocks (64
+// registers) 1806 and 1577, 5 blocks (96 registers) 1668 and 1451.
 constexpr int kMinBlocksPlain = BH_WALK_MIN_BLOCKS_PLAIN;
 constexpr int kMinBlocksRelative = BH_WALK_MIN_BLOCKS_RELATIVE;
 // 64-body groups (two bodies per lane), every criterion: 4 blocks (up to 128
@@ -82,23 +95,10 @@ __host__ __device__ constexpr int walk_min_blocks(bool relative, bool wide) {
 constexpr int kBlocksPerSm = 8;  // persistent grid: blocks launched per SM (the excess waits)
 constexpr int kSpillPerWarp = 4096;  // global stack entries per warp beyond shared memory
 constexpr float kBoxMargin = 1.0f - 1.0f / 65536.0f;
-#ifndef BH_WALK_PACKED
-#define BH_WALK_PACKED 1
-#endif
-constexpr bool kWalkPacked = BH_WALK_PACKED != 0;
-// Each lane's running force sums (and their Kahan compensations) live in
-// shared memory between list flushes instead of in registers: they are only
-// touched once per flushed list block, and the registers they free are what
-// lets more warps be resident.
-#ifndef BH_WALK_SUMS_SMEM
-#define BH_WALK_SUMS_SMEM 1
-#endif
-constexpr bool kSumsSmem = BH_WALK_SUMS_SMEM != 0;
-// Take groups in the order the caller gives (longest lists first).
-#ifndef BH_WALK_GROUP_ORDER
-#define BH_WALK_GROUP_ORDER 1
-#endif
-constexpr bool kGroupOrder = BH_WALK_GROUP_ORDER != 0;
+// nodes waiting for their representative test (fewer than 32 before a round
+// of 64 box tests) and for the exact vote (fewer than 32 before 32 more)
+constexpr int kPendCap = 96;
+constexpr int kVoteCap = 64;
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
@@ -133,6 +133,71 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     return r;
 }
 
+// min of three, for a squared distance against a bound: a NaN stays one (the
+// comparison with it then opens), or is passed over
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Shared memory by 32-bit address: one base register per warp and immediate
+// offsets.  (Through C++ arrays the compiler kept recomputing the thread's
+// indices and the window's base in every round.)
+__device__ __forceinline__ int lds_i(unsigned a) {
+    int v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float lds_f(unsigned a) { return __int_as_float(lds_i(a)); }
+__device__ __forceinline__ float4 lds_f4(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ ulonglong2 lds_2x2(unsigned a) {  // two packed pairs
+    ulonglong2 v;
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_i(unsigned a, int v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v)); }
+__device__ __forceinline__ void sts_f(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v)); }
+__device__ __forceinline__ void sts_f4(unsigned a, float4 v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+}
+
+// A warp's shared memory, byte offsets from its base:
+//   list   the interaction list as four arrays of kListCap floats: x[], y[], z[], m[]
+//   body   the group's bodies for the exact vote, in pairs: (x0, x1, y0, y1),
+//          (z0, z1, k0, k1), k the body's share of the relative criterion; a
+//          partial group is filled up with copies of its first body, which
+//          change no verdict
+//   rep    the group's representative body of each box octant, (x, y, z, k)
+//   sum    per lane: running sums x, y, z, compensations x, y, z (then the
+//          second body's): touched once per flushed list block only, and the
+//          registers they free let more warps be resident
+//   pend   nodes the box test could not accept, and
+//   vote   of those the ones no representative body opens
+//   group  the group being walked and its interaction-list length so far
+//   stack  the traversal stack's first stackSmem entries
+template <bool kWide>
+struct WarpMem {
+    static constexpr unsigned list = 0, listArray = 4u * kListCap;
+    static constexpr unsigned body = list + 4 * listArray;
+    static constexpr unsigned rep = body + 16u * (kWide ? 64 : 32);
+    static constexpr unsigned sum = rep + 16u * 8;
+    static constexpr unsigned pend = sum + 128u * (kWide ? 12 : 6);
+    static constexpr unsigned vote = pend + 4u * kPendCap;
+    static constexpr unsigned group = vote + 4u * kVoteCap;
+    static constexpr unsigned stack = group + 16;
+    static constexpr unsigned bytes(int stackSmem) { return stack + 4u * (unsigned)stackSmem; }
+};
+
 // The reference's d^2 (tree.cu:611) as its compiled walk evaluates it:
 // fma(dz, dz, fma(dx, dx, dy * dy)).  The opening test must round exactly
 // like the reference's for the interaction sets to be identical.
@@ -142,13 +207,10 @@ __device__ __forceinline__ float ref_dist_sq(float dx, float dy, float dz) {
 
 }  // namespace
 
-// One warp per group of 32 bodies (kWide: 64, two per lane).  kPacked selects
-// the interaction loop: packed FP32x2 over a component-array list, or scalar
-// FP32 over float4 entries (32-body groups only).
-template <bool kFused, bool kCompensated, bool kPacked, bool kRelative, bool kBuckets, bool kWide>
+// One warp per group of 32 bodies (kWide: 64, two per lane).
+template <bool kFused, bool kCompensated, bool kRelative, bool kBuckets, bool kWide>
 __global__ void __launch_bounds__(kThreads, walk_min_blocks(kRelative, kWide))
 k_walk(const WalkArgs a) {
-    static_assert(kPacked || !kWide, "64-body groups use the packed interaction loop");
     constexpr int kW = kWide ? 64 : 32;
     const float4* __restrict__ pos = a.pos;
     const WalkNode* __restrict__ wn = a.wn;
@@ -156,31 +218,16 @@ k_walk(const WalkArgs a) {
     const float eps2 = a.eps2, G = a.G, dt = a.dt;
     int* err = a.err;
     const int spillPerWarp = kSpillPerWarp;
-    // per-warp traversal stack: stackSmem entries per warp in dynamic shared
-    // memory, entries past them spill to global memory
-    extern __shared__ int sDynStack[];
     const int stackSmem = a.stackSmem;
-    // per-warp interaction list: float4 (x, y, z, m) per entry, or, packed,
-    // the same storage as four arrays of kListCap floats: x[], y[], z[], m[]
-    __shared__ float4 sList[kWarpsPerBlock][kListCap];
-    // the nodes a round votes on, compacted and pair-interleaved:
-    // sVote[2j] = (x_2j, x_2j+1, y_2j, y_2j+1), sVote[2j+1] = (z.., z.., size^2.., size^2..)
-    // (entries 64-65 take the writes of the nodes that are not staged, so that
-    // staging needs no branch)
-    __shared__ float4 sVote[kWarpsPerBlock][66];
-    __shared__ __align__(8) float sVoteMs[kRelative ? kWarpsPerBlock : 1][66];  // mass * size^2 of those nodes
-    // per warp: the group being walked and its interaction-list length so far
-    // (kept here rather than in registers, which the walk is short of)
-    __shared__ int sGroupLen[kWarpsPerBlock][2];
-    // per warp: the group's representative body of each box octant, (x, y, z, |a|)
-    __shared__ float4 sRep[kWarpsPerBlock][8];
-    // per lane: sums x, y, z, compensations x, y, z (then the second body's)
-    constexpr int kSums = kWide ? 12 : 6;
-    __shared__ float sSum[kSumsSmem ? kWarpsPerBlock : 1][kSumsSmem ? kSums : 1][32];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned lt = lanemask_lt();
-    int* spill = a.spill + (size_t)(blockIdx.x * kWarpsPerBlock + w) * spillPerWarp;
-    int* const sStk = sDynStack + w * stackSmem;  // this warp's stack
+    using Mem = WarpMem<kWide>;
+    constexpr unsigned kSums = kWide ? 12 : 6;
+    extern __shared__ __align__(16) char sDyn[];
+    int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    unsigned lt = lanemask_lt(), sm = (unsigned)__cvta_generic_to_shared(sDyn) + wi * Mem::bytes(stackSmem);
+    // (opaque from here on: kept in registers, not recomputed in every round)
+    asm volatile("" : "+r"(lane), "+r"(lt), "+r"(sm));
+    const unsigned sl = sm + 4u * lane;  // this lane's column
+    int* spill = a.spill + (size_t)(blockIdx.x * kWarpsPerBlock + wi) * spillPerWarp;
     const int stackCap = stackSmem + spillPerWarp;
     const int groups = a.groupTable ? a.groups : (n + kW - 1) / kW;
     const int leafSize = a.leafSize > 1 ? a.leafSize : 1;  // nodes with at most this many bodies are buckets
@@ -200,7 +247,7 @@ k_walk(const WalkArgs a) {
         int g = 0;
         if (lane == 0) {
             g = atomicAdd(&a.ctr->groupCursor, 1);
-            if (kGroupOrder && a.groupOrder && g < groups) g = a.groupOrder[g];  // longest lists first
+            if (a.groupOrder && g < groups) g = a.groupOrder[g];  // longest lists first
         }
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= groups) break;
@@ -226,8 +273,7 @@ k_walk(const WalkArgs a) {
             const float4 q = pos[b1];
             p1 = make_float3(q.x, q.y, q.z);
         }
-        int nValid = __popc(__ballot_sync(0xffffffffu, valid));
-        if (kWide) nValid += __popc(__ballot_sync(0xffffffffu, valid1));
+        const int nValid = cnt;
         // opening parameters of this group (per 32-body group; a 64-body group
         // takes the smaller theta and budget of its two halves)
         float theta = a.theta, kA = 0.f;
@@ -246,16 +292,30 @@ k_walk(const WalkArgs a) {
         const float thetaSq = __fmul_rn(theta, theta);
         const float thetaSqBox = thetaSq * kBoxMargin;
         // relative criterion: open when M s^2 > kA |a_b| d^4 for some body
-        float myA = 0.f, myA1 = 0.f, aMin = 0.f;
+        float myA = 0.f, myA1 = 0.f, kAmin = 0.f;
         if (kRelative) {
             myA = valid ? a.aMagIn[b] : INFINITY;
-            aMin = myA;
+            float aMin = myA;
             if (kWide) {
                 myA1 = valid1 ? a.aMagIn[b1] : INFINITY;
                 aMin = fminf(aMin, myA1);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) aMin = fminf(aMin, __shfl_xor_sync(0xffffffffu, aMin, o));
+            kAmin = kA * aMin * kBoxMargin;
+        }
+        {  // the bodies as the vote reads them
+            const float4 f = make_float4(__shfl_sync(0xffffffffu, p.x, 0), __shfl_sync(0xffffffffu, p.y, 0),
+                                         __shfl_sync(0xffffffffu, p.z, 0), __shfl_sync(0xffffffffu, myA, 0));
+            auto put = [&](int i, bool v, float x, float y, float z, float am) {
+                const unsigned e = sm + Mem::body + 32u * (i >> 1) + 4u * (i & 1);
+                sts_f(e, v ? x : f.x);
+                sts_f(e + 8, v ? y : f.y);
+                sts_f(e + 16, v ? z : f.z);
+                sts_f(e + 24, kRelative ? kA * (v ? am : f.w) : 0.f);
+            };
+            put(lane, valid, p.x, p.y, p.z, myA);
+            if (kWide) put(lane + 32, valid1, p1.x, p1.y, p1.z, myA1);
         }
 
         // group box as centre +- half extent; the half extent is rounded
@@ -304,7 +364,8 @@ k_walk(const WalkArgs a) {
                 }
                 const unsigned best = __reduce_min_sync(0xffffffffu, (__float_as_uint(d) & ~31u) | (unsigned)lane);
                 if ((best & 31u) == (unsigned)lane)
-                    sRep[w][o] = second ? make_float4(p1.x, p1.y, p1.z, myA1) : make_float4(p.x, p.y, p.z, myA);
+                    sts_f4(sm + Mem::rep + 16u * o, second ? make_float4(p1.x, p1.y, p1.z, kA * myA1)
+                                                           : make_float4(p.x, p.y, p.z, kA * myA));
             }
         }
 
@@ -313,427 +374,312 @@ k_walk(const WalkArgs a) {
         {
             const int rb = wn[root].childBegin, re = wn[root].childEnd;
             top = re - rb;
-            if (lane < top) sStk[lane] = rb + lane;
+            if (lane < top) sts_i(sl + Mem::stack, rb + lane);
         }
-        __syncwarp();
-        int listLen = 0;
+        int listLen = 0, pendLen = 0, voteLen = 0;
         if (lane == 0) {
-            sGroupLen[w][0] = g;
-            sGroupLen[w][1] = 0;
+            sts_i(sm + Mem::group, g);
+            sts_i(sm + Mem::group + 4, 0);
         }
-        float sx = 0.f, sy = 0.f, sz = 0.f;  // running sums
-        float cx = 0.f, cy = 0.f, cz = 0.f;  // Kahan compensation
-        float tx = 0.f, ty = 0.f, tz = 0.f;  // the second body's (64-body groups)
-        float ux = 0.f, uy = 0.f, uz = 0.f;
-        if (kSumsSmem)  // this lane's column only: no synchronisation needed
 #pragma unroll
-            for (int k = 0; k < kSums; k++) sSum[w][k][lane] = 0.f;
+        for (unsigned k = 0; k < kSums; k++) sts_f(sl + Mem::sum + 128u * k, 0.f);  // this lane's column only
+        __syncwarp();
 
         // interactions with list entries [0, cnt); partial sums Kahan-added
-        auto kahan = [&](float ax, float ay, float az, float& s0, float& s1, float& s2, float& c0, float& c1,
-                         float& c2) {
+        auto kahan = [&](float ax, float ay, float az, unsigned S) {
+            float s0 = lds_f(S), s1 = lds_f(S + 128), s2 = lds_f(S + 256);
             if (kCompensated) {
+                float c0 = lds_f(S + 384), c1 = lds_f(S + 512), c2 = lds_f(S + 640);
                 float y, t;
                 y = ax - c0; t = s0 + y; c0 = (t - s0) - y; s0 = t;
                 y = ay - c1; t = s1 + y; c1 = (t - s1) - y; s1 = t;
                 y = az - c2; t = s2 + y; c2 = (t - s2) - y; s2 = t;
+                sts_f(S + 384, c0);
+                sts_f(S + 512, c1);
+                sts_f(S + 640, c2);
             } else {
                 s0 += ax; s1 += ay; s2 += az;
             }
+            sts_f(S, s0);
+            sts_f(S + 128, s1);
+            sts_f(S + 256, s2);
         };
         auto flush = [&](int cnt) {
             float ax, ay, az;
             float bx = 0.f, by = 0.f, bz = 0.f;  // second body (64-body groups)
-            if (kPacked) {
-                // the list as four component arrays x[], y[], z[], m[]: one
-                // 16-byte load gives four entries' x, i.e. two packed pairs
-                const float* L = reinterpret_cast<const float*>(sList[w]);
-                const ulonglong2* X = reinterpret_cast<const ulonglong2*>(L);
-                const ulonglong2* Y = reinterpret_cast<const ulonglong2*>(L + kListCap);
-                const ulonglong2* Z = reinterpret_cast<const ulonglong2*>(L + 2 * kListCap);
-                const ulonglong2* Mq = reinterpret_cast<const ulonglong2*>(L + 3 * kListCap);
-                const f32x2 px2 = pack2(p.x, p.x), py2 = pack2(p.y, p.y), pz2 = pack2(p.z, p.z);
-                const f32x2 qx2 = pack2(p1.x, p1.x), qy2 = pack2(p1.y, p1.y), qz2 = pack2(p1.z, p1.z);
-                const f32x2 e2 = pack2(eps2, eps2);
-                const int quads = cnt >> 2;
-                f32x2 ax2 = 0ull, ay2 = 0ull, az2 = 0ull;
-                f32x2 bx2 = 0ull, by2 = 0ull, bz2 = 0ull;
-                // one packed body-pair interaction: (bx, by, bz) against two entries
-                auto pair = [&](f32x2 ex, f32x2 ey, f32x2 ez, f32x2 em, f32x2 ox, f32x2 oy, f32x2 oz, f32x2& sx2,
-                                f32x2& sy2, f32x2& sz2) {
-                    const f32x2 dx = sub2(ex, ox), dy = sub2(ey, oy), dz = sub2(ez, oz);
-                    f32x2 r2 = fma2(dx, dx, e2);
-                    r2 = fma2(dy, dy, r2);
-                    r2 = fma2(dz, dz, r2);
-                    float r2a, r2b;
-                    unpack2(r2, r2a, r2b);
-                    const f32x2 ri = pack2(rsqrt_approx(r2a), rsqrt_approx(r2b));
-                    const f32x2 f = mul2(mul2(em, ri), mul2(ri, ri));
-                    sx2 = fma2(f, dx, sx2);
-                    sy2 = fma2(f, dy, sy2);
-                    sz2 = fma2(f, dz, sz2);
-                };
-                if (kWide) {
+            // one 16-byte load of a component array gives four entries' x,
+            // i.e. two packed pairs
+            const f32x2 px2 = pack2(p.x, p.x), py2 = pack2(p.y, p.y), pz2 = pack2(p.z, p.z);
+            const f32x2 qx2 = pack2(p1.x, p1.x), qy2 = pack2(p1.y, p1.y), qz2 = pack2(p1.z, p1.z);
+            const f32x2 e2 = pack2(eps2, eps2);
+            const unsigned end = sm + 4u * cnt;  // cnt is a multiple of 32
+            f32x2 ax2 = 0ull, ay2 = 0ull, az2 = 0ull;
+            f32x2 bx2 = 0ull, by2 = 0ull, bz2 = 0ull;
+            // one packed body-pair interaction: (bx, by, bz) against two entries
+            auto pair = [&](f32x2 ex, f32x2 ey, f32x2 ez, f32x2 em, f32x2 ox, f32x2 oy, f32x2 oz, f32x2& sx2,
+                            f32x2& sy2, f32x2& sz2) {
+                const f32x2 dx = sub2(ex, ox), dy = sub2(ey, oy), dz = sub2(ez, oz);
+                f32x2 r2 = fma2(dx, dx, e2);
+                r2 = fma2(dy, dy, r2);
+                r2 = fma2(dz, dz, r2);
+                float r2a, r2b;
+                unpack2(r2, r2a, r2b);
+                const f32x2 ri = pack2(rsqrt_approx(r2a), rsqrt_approx(r2b));
+                const f32x2 f = mul2(mul2(em, ri), mul2(ri, ri));
+                sx2 = fma2(f, dx, sx2);
+                sy2 = fma2(f, dy, sy2);
+                sz2 = fma2(f, dz, sz2);
+            };
+            auto quad = [&](unsigned L) {  // four list entries
+                const ulonglong2 x = lds_2x2(L), y = lds_2x2(L + Mem::listArray);
+                const ulonglong2 z = lds_2x2(L + 2 * Mem::listArray), m = lds_2x2(L + 3 * Mem::listArray);
+                pair(x.x, y.x, z.x, m.x, px2, py2, pz2, ax2, ay2, az2);
+                if (kWide) pair(x.x, y.x, z.x, m.x, qx2, qy2, qz2, bx2, by2, bz2);
+                pair(x.y, y.y, z.y, m.y, px2, py2, pz2, ax2, ay2, az2);
+                if (kWide) pair(x.y, y.y, z.y, m.y, qx2, qy2, qz2, bx2, by2, bz2);
+            };
+            constexpr unsigned kQuads = kWide ? 2 : 8;
 #pragma unroll 1
-                    for (int k = 0; k < quads; k++) {
-                        const ulonglong2 x = X[k], y = Y[k], z = Z[k], m = Mq[k];
-                        pair(x.x, y.x, z.x, m.x, px2, py2, pz2, ax2, ay2, az2);
-                        pair(x.x, y.x, z.x, m.x, qx2, qy2, qz2, bx2, by2, bz2);
-                        pair(x.y, y.y, z.y, m.y, px2, py2, pz2, ax2, ay2, az2);
-                        pair(x.y, y.y, z.y, m.y, qx2, qy2, qz2, bx2, by2, bz2);
-                    }
-                } else {
-#pragma unroll 8
-                    for (int k = 0; k < quads; k++) {
-                        const ulonglong2 x = X[k], y = Y[k], z = Z[k], m = Mq[k];
-                        pair(x.x, y.x, z.x, m.x, px2, py2, pz2, ax2, ay2, az2);
-                        pair(x.y, y.y, z.y, m.y, px2, py2, pz2, ax2, ay2, az2);
-                    }
-                }
-                if (cnt & 2) {  // a pair left over
-                    const int j = 4 * quads;
-                    const f32x2 x = *reinterpret_cast<const f32x2*>(L + j);
-                    const f32x2 y = *reinterpret_cast<const f32x2*>(L + kListCap + j);
-                    const f32x2 z = *reinterpret_cast<const f32x2*>(L + 2 * kListCap + j);
-                    const f32x2 m = *reinterpret_cast<const f32x2*>(L + 3 * kListCap + j);
-                    pair(x, y, z, m, px2, py2, pz2, ax2, ay2, az2);
-                    if (kWide) pair(x, y, z, m, qx2, qy2, qz2, bx2, by2, bz2);
-                }
-                float a0, a1;
-                unpack2(ax2, a0, a1);
-                ax = a0 + a1;
-                unpack2(ay2, a0, a1);
-                ay = a0 + a1;
-                unpack2(az2, a0, a1);
-                az = a0 + a1;
-                if (kWide) {
-                    unpack2(bx2, a0, a1);
-                    bx = a0 + a1;
-                    unpack2(by2, a0, a1);
-                    by = a0 + a1;
-                    unpack2(bz2, a0, a1);
-                    bz = a0 + a1;
-                }
-                if (cnt & 1) {  // the last entry alone
-                    const int j = cnt - 1;
-                    const float ex = L[j], ey = L[kListCap + j], ez = L[2 * kListCap + j], em = L[3 * kListCap + j];
-                    auto one = [&](float ox, float oy, float oz, float& rx, float& ry, float& rz) {
-                        const float dx = ex - ox, dy = ey - oy, dz = ez - oz;
-                        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, eps2)));
-                        const float ri = rsqrt_approx(r2);
-                        const float f = (em * ri) * (ri * ri);
-                        rx = __fmaf_rn(f, dx, rx);
-                        ry = __fmaf_rn(f, dy, ry);
-                        rz = __fmaf_rn(f, dz, rz);
-                    };
-                    one(p.x, p.y, p.z, ax, ay, az);
-                    if (kWide) one(p1.x, p1.y, p1.z, bx, by, bz);
-                }
-            } else {
-                float hx = 0.f, hy = 0.f, hz = 0.f;
-                ax = ay = az = 0.f;
-                int k = 0;
-                for (; k + 1 < cnt; k += 2) {  // two independent chains
-                    const float4 c0 = sList[w][k], c1 = sList[w][k + 1];
-                    const float dx0 = c0.x - p.x, dy0 = c0.y - p.y, dz0 = c0.z - p.z;
-                    const float dx1 = c1.x - p.x, dy1 = c1.y - p.y, dz1 = c1.z - p.z;
-                    const float r0 = __fmaf_rn(dz0, dz0, __fmaf_rn(dy0, dy0, __fmaf_rn(dx0, dx0, eps2)));
-                    const float r1 = __fmaf_rn(dz1, dz1, __fmaf_rn(dy1, dy1, __fmaf_rn(dx1, dx1, eps2)));
-                    const float i0 = rsqrt_approx(r0), i1 = rsqrt_approx(r1);
-                    const float f0 = (c0.w * i0) * (i0 * i0), f1 = (c1.w * i1) * (i1 * i1);
-                    ax = __fmaf_rn(f0, dx0, ax);
-                    hx = __fmaf_rn(f1, dx1, hx);
-                    ay = __fmaf_rn(f0, dy0, ay);
-                    hy = __fmaf_rn(f1, dy1, hy);
-                    az = __fmaf_rn(f0, dz0, az);
-                    hz = __fmaf_rn(f1, dz1, hz);
-                }
-                if (k < cnt) {
-                    const float4 c = sList[w][k];
-                    const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
-                    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, eps2)));
-                    const float ri = rsqrt_approx(r2);
-                    const float f = (c.w * ri) * (ri * ri);
-                    ax = __fmaf_rn(f, dx, ax);
-                    ay = __fmaf_rn(f, dy, ay);
-                    az = __fmaf_rn(f, dz, az);
-                }
-                ax += hx;
-                ay += hy;
-                az += hz;
+            for (unsigned L = sm; L < end; L += 16 * kQuads)
+#pragma unroll
+                for (unsigned k = 0; k < kQuads; k++) quad(L + 16 * k);
+            float a0, a1;
+            unpack2(ax2, a0, a1);
+            ax = a0 + a1;
+            unpack2(ay2, a0, a1);
+            ay = a0 + a1;
+            unpack2(az2, a0, a1);
+            az = a0 + a1;
+            if (kWide) {
+                unpack2(bx2, a0, a1);
+                bx = a0 + a1;
+                unpack2(by2, a0, a1);
+                by = a0 + a1;
+                unpack2(bz2, a0, a1);
+                bz = a0 + a1;
             }
-            if (kSumsSmem) {
-                float (*S)[32] = sSum[w];
-                float s0 = S[0][lane], s1 = S[1][lane], s2 = S[2][lane];
-                float c0 = S[3][lane], c1 = S[4][lane], c2 = S[5][lane];
-                kahan(ax, ay, az, s0, s1, s2, c0, c1, c2);
-                S[0][lane] = s0; S[1][lane] = s1; S[2][lane] = s2;
-                S[3][lane] = c0; S[4][lane] = c1; S[5][lane] = c2;
-                if (kWide) {
-                    float t0 = S[kSums - 6][lane], t1 = S[kSums - 5][lane], t2 = S[kSums - 4][lane];
-                    float u0 = S[kSums - 3][lane], u1 = S[kSums - 2][lane], u2 = S[kSums - 1][lane];
-                    kahan(bx, by, bz, t0, t1, t2, u0, u1, u2);
-                    S[kSums - 6][lane] = t0; S[kSums - 5][lane] = t1; S[kSums - 4][lane] = t2;
-                    S[kSums - 3][lane] = u0; S[kSums - 2][lane] = u1; S[kSums - 1][lane] = u2;
-                }
-            } else {
-                kahan(ax, ay, az, sx, sy, sz, cx, cy, cz);
-                if (kWide) kahan(bx, by, bz, tx, ty, tz, ux, uy, uz);
-            }
+            kahan(ax, ay, az, sl + Mem::sum);
+            if (kWide) kahan(bx, by, bz, sl + Mem::sum + 128u * (kSums - 6));
         };
 
-        // One round tests up to 64 nodes, two per lane (slot 0 from the top 32
-        // stack entries, slot 1 from the next 32).
         // A stack entry is a node index (>= 0) or, below a bucket node that
         // was opened, a body b encoded as -(b + 2): a body is a leaf, always
-        // accepted.  Slot index -1 is an idle slot.
-        struct Slot {
-            int idx;
-            float4 com;
-            int cb, ce;
-            float sizeSq;
-            int count;
-            bool open, undecided;
+        // accepted.
+        auto popped = [&](int at) -> int {
+            return at < stackSmem ? lds_i(sm + Mem::stack + 4u * at) : spill[at - stackSmem];
         };
-        auto load = [&](Slot& t, int stackPos, bool has) {
-            t.idx = -1;
-            if (has) t.idx = (stackPos < stackSmem) ? sStk[stackPos] : spill[stackPos - stackSmem];
-            t.count = 0;
-            if (!kBuckets) {
-                // every lane loads a record (an idle slot the root's) and an
-                // idle slot gets an empty child range: no branch
-                const int li = t.idx >= 0 ? t.idx : 0;
-                t.com = wn[li].com;
-                const int4 meta = *reinterpret_cast<const int4*>(&wn[li].childBegin);
-                t.cb = meta.x;
-                t.ce = t.idx >= 0 ? meta.y : meta.x;
-                t.sizeSq = __int_as_float(meta.z);
-                return;
-            }
-            t.com = make_float4(0.f, 0.f, 0.f, 0.f);
-            t.cb = t.ce = 0;
-            t.sizeSq = 0.f;
-            if (t.idx >= 0) {
-                t.com = wn[t.idx].com;
-                const int4 meta = *reinterpret_cast<const int4*>(&wn[t.idx].childBegin);
-                t.cb = meta.x;
-                t.ce = meta.y;
-                t.sizeSq = __int_as_float(meta.z);
-                t.count = meta.w;
-            } else if (t.idx < -1) {
-                t.com = pos[-t.idx - 2];
-                t.count = 1;
-            }
+        auto append = [&](const float4& com, bool accept, int k) {
+            if (!accept) return;  // component arrays: consecutive entries, conflict-free stores
+            const unsigned L = sm + 4u * k;
+            sts_f(L, com.x);
+            sts_f(L + Mem::listArray, com.y);
+            sts_f(L + 2 * Mem::listArray, com.z);
+            sts_f(L + 3 * Mem::listArray, com.w);
         };
-        auto classify = [&](Slot& t) {
-            // every test computed for every slot, combined without branches
-            const bool internal = t.cb != t.ce;  // leaves and idle slots have cb == ce
-            const float gx = fmaxf(fabsf(t.com.x - bm[0]) - be[0], 0.f);
-            const float gy = fmaxf(fabsf(t.com.y - bm[1]) - be[1], 0.f);
-            const float gz = fmaxf(fabsf(t.com.z - bm[2]) - be[2], 0.f);
+        // The box test of one stack entry: true when it is a leaf, a body or
+        // far enough from the whole group, false when it needs a closer look.
+        auto closed = [&](int idx, float4& com) -> bool {
+            const int li = kBuckets && idx < 0 ? 0 : idx;
+            com = wn[li].com;
+            const int4 meta = *reinterpret_cast<const int4*>(&wn[li].childBegin);
+            if (kBuckets && idx < 0) com = pos[-idx - 2];
+            const float gx = fmaxf(fabsf(com.x - bm[0]) - be[0], 0.f);
+            const float gy = fmaxf(fabsf(com.y - bm[1]) - be[1], 0.f);
+            const float gz = fmaxf(fabsf(com.z - bm[2]) - be[2], 0.f);
             const float D2 = gx * gx + gy * gy + gz * gz;
-            bool boxAccept = thetaSqBox * D2 > t.sizeSq;
-            if (kRelative) boxAccept = boxAccept && (t.com.w * t.sizeSq < kA * aMin * (D2 * D2) * kBoxMargin);
-            const int oc = (t.com.x > bm[0] ? 4 : 0) | (t.com.y > bm[1] ? 2 : 0) | (t.com.z > bm[2] ? 1 : 0);
-            const float4 r = sRep[w][oc];  // (x, y, z, |a|) of the octant's representative
-            const float d2 = ref_dist_sq(r.x - t.com.x, r.y - t.com.y, r.z - t.com.z);
-            bool repOpen = !(t.sizeSq < __fmul_rn(thetaSq, d2));
-            if (kRelative) repOpen = repOpen || (t.com.w * t.sizeSq > kA * r.w * (d2 * d2));
-            t.open = internal && !boxAccept && repOpen;
-            t.undecided = internal && !boxAccept && !repOpen;
-        };
-        auto append = [&](const Slot& t, bool accept, int k) {
-            if (!accept) return;
-            if (kPacked) {  // component arrays: consecutive entries, conflict-free stores
-                float* L = reinterpret_cast<float*>(sList[w]);
-                L[k] = t.com.x;
-                L[kListCap + k] = t.com.y;
-                L[2 * kListCap + k] = t.com.z;
-                L[3 * kListCap + k] = t.com.w;
-            } else {
-                sList[w][k] = t.com;
-            }
-        };
-        // entries an opened node puts on the stack: its children (next level,
-        // at most 8; anything else is a broken tree, reported rather than
-        // followed) or, for a bucket (at most leafSize bodies), its bodies.
-        // first: the first pushed value; entries are first + c (children) or
-        // first - c (bodies, encoded).
-        auto children = [&](const Slot& t, int& first, int& stepSign) -> int {
-            first = t.cb;
-            stepSign = 1;
-            if (!t.open) return 0;
-            if (kBuckets && t.count <= leafSize) {
-                first = -(a.nFirst[t.idx] + 2);
-                stepSign = -1;
-                return t.count;
-            }
-            const int c = t.ce - t.cb;
-            if (t.cb <= t.idx || c > 8) {
-                bh_set_error(err, BH_ERR_INTERNAL);
-                return 0;
-            }
+            const float sizeSq = __int_as_float(meta.z);
+            bool c = thetaSqBox * D2 > sizeSq;
+            if (kRelative) c = c & (com.w * sizeSq < kAmin * (D2 * D2));
+            c = c | (meta.x == meta.y);  // a leaf never opens
+            if (kBuckets) c = c | (idx < 0);
             return c;
-        };
-        auto push = [&](int pos, int v) {
-            if (pos < stackSmem) sStk[pos] = v;
-            else spill[pos - stackSmem] = v;
         };
 
         bool overflow = false;
-        while (top > 0) {
-            const int take = top < 64 ? top : 64;
-            top -= take;
-            Slot s0, s1;
-            load(s0, top + lane, lane < take);
-            load(s1, top + 32 + lane, 32 + lane < take);
-            __syncwarp();
-            classify(s0);
-            classify(s1);
-            // exact group vote for the undecided nodes (tree.cu:629-640)
-            unsigned und0 = __ballot_sync(0xffffffffu, s0.undecided);
-            unsigned und1 = __ballot_sync(0xffffffffu, s1.undecided);
-            if (und0 | und1) {
-                // compact the undecided nodes (those of slot 0, then of slot 1)
-                // pair-interleaved, so that one pass
-                // tests two nodes with packed FP32x2 arithmetic; every packed
-                // operation rounds exactly like the scalar one it replaces
-                const int c0 = __popc(und0), u = c0 + __popc(und1);
-                nVote += u;
-                const int k0 = __popc(und0 & lt), k1 = c0 + __popc(und1 & lt);
-                auto stage = [&](const Slot& t, int k) {
-                    float* e = reinterpret_cast<float*>(&sVote[w][2 * (k >> 1)]) + (k & 1);
-                    e[0] = t.com.x;
-                    e[2] = t.com.y;
-                    e[4] = t.com.z;
-                    e[6] = t.sizeSq;
-                    if (kRelative) sVoteMs[w][k] = t.com.w * t.sizeSq;
-                };
-                stage(s0, s0.undecided ? k0 : 64);
-                stage(s1, s1.undecided ? k1 : 64);
-                __syncwarp();
-                const ulonglong2* V = reinterpret_cast<const ulonglong2*>(sVote[w]);
-                const f32x2 th2 = pack2(thetaSq, thetaSq);
-                const float kAa = kA * myA, kAa1 = kA * myA1;
-                // which of the two staged nodes a body at (x, y, z) wants opened
-                auto wants2 = [&](ulonglong2 xy, ulonglong2 zs, f32x2 ms, float bx, float by, float bz, float ka,
-                                  bool& wa, bool& wb) {
-                    const f32x2 dx = sub2(pack2(bx, bx), xy.x), dy = sub2(pack2(by, by), xy.y);
-                    const f32x2 dz = sub2(pack2(bz, bz), zs.x);
-                    const f32x2 d2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));  // ref_dist_sq, packed
-                    float ta, tb, sa, sb;
-                    unpack2(mul2(th2, d2), ta, tb);
-                    unpack2(zs.y, sa, sb);
-                    wa = !(sa < ta);
-                    wb = !(sb < tb);
-                    if (kRelative) {
-                        float ra, rb, ma, mb;
-                        unpack2(mul2(pack2(ka, ka), mul2(d2, d2)), ra, rb);
-                        unpack2(ms, ma, mb);
-                        wa = wa || (ma > ra);
-                        wb = wb || (mb > rb);
-                    }
-                };
-                // each lane collects its own body's wishes, bit j for staged node
-                // j; one warp OR per 32 staged nodes then gives the verdicts
-                // (1% faster than an OR after every pass)
-                unsigned long long mine = 0ull;
-#pragma unroll 2
-                for (int j = 0; j < u; j += 2) {
-                    const ulonglong2 xy = V[j], zs = V[j + 1];
-                    f32x2 ms = 0ull;
-                    if (kRelative) ms = *reinterpret_cast<const f32x2*>(&sVoteMs[w][j]);
-                    bool wa, wb;
-                    wants2(xy, zs, ms, p.x, p.y, p.z, kAa, wa, wb);
-                    wa = valid && wa;
-                    wb = valid && wb;
-                    if (kWide) {
-                        bool va, vb;
-                        wants2(xy, zs, ms, p1.x, p1.y, p1.z, kAa1, va, vb);
-                        wa = wa || (valid1 && va);
-                        wb = wb || (valid1 && vb);
-                    }
-                    mine |= (unsigned long long)((wa ? 1u : 0u) | (wb ? 2u : 0u)) << j;
+        for (;;) {
+            // (a round of fewer than 32 entries waits until nothing else is
+            // left to do: 152 against 157 us at 16,384 bodies, large walks the same)
+            if ((top >= 32 || (top > 0 && (pendLen | voteLen) == 0)) && (pendLen | voteLen) < 32) {
+                // ---- box tests of up to 64 stack entries, two per lane
+                const int take = top < 64 ? top : 64;
+                top -= take;
+                const bool h0 = lane < take, h1 = lane + 32 < take;
+                int i0 = 0, i1 = 0;
+                if (top + 64 <= stackSmem) {  // uniform: the usual case
+                    const unsigned q = sl + Mem::stack + 4u * top;
+                    i0 = lds_i(q);
+                    i1 = lds_i(q + 128);
+                    i0 = h0 ? i0 : 0;
+                    i1 = h1 ? i1 : 0;
+                } else {
+                    if (h0) i0 = popped(top + lane);
+                    if (h1) i1 = popped(top + 32 + lane);
                 }
-                // an odd count leaves the last pair's second half stale: masked
-                const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)mine);
-                const unsigned hi = u > 32 ? __reduce_or_sync(0xffffffffu, (unsigned)(mine >> 32)) : 0u;
-                unsigned long long openedC = ((unsigned long long)hi << 32) | lo;
-                if (u < 64) openedC &= (1ull << u) - 1ull;
-                s0.open = s0.open || (s0.undecided && ((openedC >> k0) & 1ull));
-                s1.open = s1.open || (s1.undecided && ((openedC >> k1) & 1ull));
-                __syncwarp();
-            }
-            const bool acc0 = (kBuckets ? s0.idx != -1 : s0.idx >= 0) && !s0.open;
-            const bool acc1 = (kBuckets ? s1.idx != -1 : s1.idx >= 0) && !s1.open;
-            const unsigned am0 = __ballot_sync(0xffffffffu, acc0), am1 = __ballot_sync(0xffffffffu, acc1);
-            nTested += take;
-            append(s0, acc0, listLen + __popc(am0 & lt));
-            append(s1, acc1, listLen + __popc(am0) + __popc(am1 & lt));
-            listLen += __popc(am0) + __popc(am1);
-            // opened nodes -> children (or a bucket's bodies) onto the stack
-            int f0, f1, d0, d1;
-            const int n0 = children(s0, f0, d0), n1 = children(s1, f1, d1);
-            int incl = n0 + n1;
+                float4 c0, c1;
+                const bool cl0 = closed(i0, c0), cl1 = closed(i1, c1);
+                const bool acc0 = h0 & cl0, acc1 = h1 & cl1, pe0 = h0 & !cl0, pe1 = h1 & !cl1;
+                const unsigned am0 = __ballot_sync(0xffffffffu, acc0), am1 = __ballot_sync(0xffffffffu, acc1);
+                // (every entry below an entry that is pending is either
+                // accepted or pending: the ranks of the one give the other's)
+                const int r0 = __popc(am0 & lt), r1 = __popc(am1 & lt), n0 = __popc(am0), n1 = __popc(am1);
+                const int k0 = (take < 32 ? take : 32) - n0;
+                append(c0, acc0, listLen + r0);
+                append(c1, acc1, listLen + n0 + r1);
+                if (pe0) sts_i(sl + Mem::pend + 4u * (pendLen - r0), i0);
+                if (pe1) sts_i(sl + Mem::pend + 4u * (pendLen + k0 - r1), i1);
+                listLen += n0 + n1;
+                pendLen += take - n0 - n1;
+                nTested += take;
+            } else {
+                // ---- 32 pending nodes (fewer once the stack is empty), one
+                // per lane: against a representative body, or by the exact vote
+                const bool vote = voteLen >= 32 || pendLen == 0;
+                int len = vote ? voteLen : pendLen;
+                if (len == 0) break;
+                const int take = len < 32 ? len : 32;
+                len -= take;
+                const bool has = lane < take;
+                int idx = 0;
+                if (has) idx = lds_i(sl + (vote ? Mem::vote : Mem::pend) + 4u * len);
+                if (vote) voteLen = len;
+                else pendLen = len;
+                const float4 com = wn[idx].com;
+                const int4 meta = *reinterpret_cast<const int4*>(&wn[idx].childBegin);
+                const float sizeSq = __int_as_float(meta.z);
+                const float ms = com.w * sizeSq;
+                bool open = false;
+                if (vote) {
+                    // the reference's group vote (tree.cu:629-640): open when
+                    // any body of the group fails; two bodies per pass, every
+                    // packed operation rounding like the scalar one
+                    const f32x2 nx = pack2(com.x, com.x), ny = pack2(com.y, com.y), nz = pack2(com.z, com.z);
+                    const f32x2 th2 = pack2(thetaSq, thetaSq);
+                    // any body fails: the nearest does (rounding is monotonic)
+                    float tMin = INFINITY, rMin = INFINITY;
+#pragma unroll 4
+                    for (unsigned B = sm + Mem::body; B < sm + Mem::body + 16u * kW; B += 32) {
+                        const ulonglong2 xy = lds_2x2(B), zk = lds_2x2(B + 16);
+                        const f32x2 dx = sub2(xy.x, nx), dy = sub2(xy.y, ny), dz = sub2(zk.x, nz);
+                        const f32x2 d2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));  // ref_dist_sq, packed
+                        float ta, tb;
+                        unpack2(mul2(th2, d2), ta, tb);
+                        tMin = min3_nan(tMin, ta, tb);
+                        if (kRelative) {
+                            float ra, rb;
+                            unpack2(mul2(zk.y, mul2(d2, d2)), ra, rb);
+                            rMin = min3(rMin, ra, rb);
+                        }
+                    }
+                    open = !(sizeSq < tMin);
+                    if (kRelative) open = open | (ms > rMin);
+                    open = open & has;
+                    const bool acc = has & !open;
+                    const unsigned am = __ballot_sync(0xffffffffu, acc);
+                    append(com, acc, listLen + __popc(am & lt));
+                    listLen += __popc(am);
+                    nVote += take;
+                } else {
+                    const int oc = (com.x > bm[0] ? 4 : 0) | (com.y > bm[1] ? 2 : 0) | (com.z > bm[2] ? 1 : 0);
+                    const float4 r = lds_f4(sm + Mem::rep + 16u * oc);  // (x, y, z, kA |a|) of the octant's representative
+                    const float d2 = ref_dist_sq(r.x - com.x, r.y - com.y, r.z - com.z);
+                    open = !(sizeSq < __fmul_rn(thetaSq, d2));
+                    if (kRelative) open = open | (ms > r.w * (d2 * d2));
+                    open = open & has;
+                    const bool un = has & !open;
+                    const unsigned um = __ballot_sync(0xffffffffu, un);
+                    if (un) sts_i(sm + Mem::vote + 4u * (voteLen + __popc(um & lt)), idx);
+                    voteLen += __popc(um);
+                }
+                // opened nodes -> their children (next level, at most 8;
+                // anything else is a broken tree, reported rather than
+                // followed) or, for a bucket (at most leafSize bodies), its
+                // bodies: entries f + d * c, c < cnt
+                int f = meta.x, d = 1, c = 0;
+                if (open) {
+                    c = meta.y - meta.x;
+                    if (kBuckets && meta.w <= leafSize) {
+                        f = -(a.nFirst[idx] + 2);
+                        d = -1;
+                        c = meta.w;
+                    } else if (meta.x <= idx || c > 8) {
+                        bh_set_error(err, BH_ERR_INTERNAL);
+                        c = 0;
+                    }
+                }
+                int incl = c;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const int pushed = __shfl_sync(0xffffffffu, incl, 31);
-            if (pushed) {
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int pushed = __shfl_sync(0xffffffffu, incl, 31);
                 if (top + pushed > stackCap) {
                     overflow = true;
                     break;
                 }
-                const int base0 = top + incl - n0 - n1, base1 = base0 + n0;
+                const int base = top + incl - c;
                 if (top + pushed <= stackSmem) {  // uniform: the usual case
-                    // at most 8 entries per slot here (a bucket holds at most
-                    // leafSize bodies; kBuckets walks take the loop below)
-                    int* q0 = &sStk[base0];
-                    int* q1 = &sStk[base1];
+                    const unsigned q = sm + Mem::stack + 4u * base;
                     if (kBuckets && leafSize > 8) {
-                        const int w0 = __reduce_max_sync(0xffffffffu, n0), w1 = __reduce_max_sync(0xffffffffu, n1);
-                        for (int c = 0; c < w0; c++)
-                            if (c < n0) q0[c] = f0 + d0 * c;
-                        for (int c = 0; c < w1; c++)
-                            if (c < n1) q1[c] = f1 + d1 * c;
+                        const int most = __reduce_max_sync(0xffffffffu, c);
+                        for (int k = 0; k < most; k++)
+                            if (k < c) sts_i(q + 4u * k, f + d * k);
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 8; c++) {  // predicated, no loop
-                            if (c < n0) q0[c] = f0 + d0 * c;
-                            if (c < n1) q1[c] = f1 + d1 * c;
-                        }
+                        for (int k = 0; k < 8; k++)  // predicated, no loop
+                            if (k < c) sts_i(q + 4u * k, kBuckets ? f + d * k : f + k);
                     }
                 } else {
-                    for (int c = 0; c < n0; c++) push(base0 + c, f0 + d0 * c);
-                    for (int c = 0; c < n1; c++) push(base1 + c, f1 + d1 * c);
+                    for (int k = 0; k < c; k++) {
+                        const int at = base + k, v = f + d * k;
+                        if (at < stackSmem) sts_i(sm + Mem::stack + 4u * at, v);
+                        else spill[at - stackSmem] = v;
+                    }
                 }
                 top += pushed;
                 maxTop = top > maxTop ? top : maxTop;
             }
             __syncwarp();
             if (listLen > kListCap - 64) {
-                flush(listLen);
-                countInteractions(listLen, nValid);
-                if (lane == 0) sGroupLen[w][1] += listLen;
-                listLen = 0;
+                // the whole blocks of 32 entries; what is left moves to the front
+                const int whole = listLen & ~31;
+                flush(whole);
+                countInteractions(whole, nValid);
+                if (lane == 0) sts_i(sm + Mem::group + 4, lds_i(sm + Mem::group + 4) + whole);
+                listLen -= whole;
+                const bool left = lane < listLen;
+                const unsigned L = left ? sl + 4u * whole : sm;
+                const float4 e = make_float4(lds_f(L), lds_f(L + Mem::listArray), lds_f(L + 2 * Mem::listArray),
+                                             lds_f(L + 3 * Mem::listArray));
+                __syncwarp();
+                append(e, left, lane);
                 __syncwarp();
             }
         }
         if (overflow && lane == 0) bh_set_error(err, BH_ERR_STACK_OVERFLOW);
         if (listLen > 0) {
-            flush(listLen);
+            // the last block, filled up with massless copies of its last entry
+            // (they add zero wherever that entry's own term is finite)
+            const int whole = (listLen + 31) & ~31;
+            const unsigned L = sm + 4u * (listLen - 1);
+            append(make_float4(lds_f(L), lds_f(L + Mem::listArray), lds_f(L + 2 * Mem::listArray), 0.f),
+                   listLen + lane < whole, listLen + lane);
+            __syncwarp();
+            flush(whole);
             countInteractions(listLen, nValid);
-            if (lane == 0) sGroupLen[w][1] += listLen;
+            if (lane == 0) sts_i(sm + Mem::group + 4, lds_i(sm + Mem::group + 4) + listLen);
         }
-        if (a.groupLen && lane == 0) a.groupLen[sGroupLen[w][0]] = sGroupLen[w][1];
+        if (a.groupLen && lane == 0) a.groupLen[lds_i(sm + Mem::group)] = lds_i(sm + Mem::group + 4);
         __syncwarp();
         // results of one body: acceleration, |a|, and the fused kick-drift
-        auto finish = [&](int bi, float bx, float by, float bz, float bm_, float s0, float s1, float s2, float c0,
-                          float c1, float c2) {
-            float gx = G * s0, gy = G * s1, gz = G * s2;
-            if (kCompensated) { gx = G * (s0 - c0); gy = G * (s1 - c1); gz = G * (s2 - c2); }
+        auto finish = [&](int bi, float bx, float by, float bz, float bm_, unsigned S) {
+            float gx = lds_f(S), gy = lds_f(S + 128), gz = lds_f(S + 256);
+            if (kCompensated) {
+                gx -= lds_f(S + 384);
+                gy -= lds_f(S + 512);
+                gz -= lds_f(S + 640);
+            }
+            gx *= G; gy *= G; gz *= G;
             if (a.accOut) a.accOut[bi] = make_float3(gx, gy, gz);
             if (a.aMagOut) a.aMagOut[bi] = sqrtf(gx * gx + gy * gy + gz * gz);
             if (kFused) {
@@ -751,17 +697,8 @@ k_walk(const WalkArgs a) {
                 }
             }
         };
-        if (kSumsSmem) {
-            const float (*S)[32] = sSum[w];
-            sx = S[0][lane]; sy = S[1][lane]; sz = S[2][lane];
-            cx = S[3][lane]; cy = S[4][lane]; cz = S[5][lane];
-            if (kWide) {
-                tx = S[kSums - 6][lane]; ty = S[kSums - 5][lane]; tz = S[kSums - 4][lane];
-                ux = S[kSums - 3][lane]; uy = S[kSums - 2][lane]; uz = S[kSums - 1][lane];
-            }
-        }
-        if (valid) finish(b, p.x, p.y, p.z, p.w, sx, sy, sz, cx, cy, cz);
-        if (kWide && valid1) finish(b1, p1.x, p1.y, p1.z, pos[b1].w, tx, ty, tz, ux, uy, uz);
+        if (valid) finish(b, p.x, p.y, p.z, p.w, sl + Mem::sum);
+        if (kWide && valid1) finish(b1, p1.x, p1.y, p1.z, pos[b1].w, sl + Mem::sum + 128u * (kSums - 6));
     }
     if (lane == 0) {
         atomicAdd(&a.ctr->interactions, (unsigned long long)nInteract);
@@ -882,8 +819,8 @@ size_t bh_walk_spill_ints() { return (size_t)bh_walk_grid() * kWarpsPerBlock * k
 // whichever binds first, never more than the register budget the variant was
 // compiled for).
 template <typename Kernel>
-static cudaError_t launch_walk_variant(Kernel kernel, const WalkArgs& a, int maxBlocks, cudaStream_t s) {
-    const size_t dyn = (size_t)kWarpsPerBlock * (size_t)a.stackSmem * sizeof(int);
+static cudaError_t launch_walk_variant(Kernel kernel, const WalkArgs& a, int maxBlocks, bool wide, cudaStream_t s) {
+    const size_t dyn = (size_t)kWarpsPerBlock * (wide ? WarpMem<true>::bytes(a.stackSmem) : WarpMem<false>::bytes(a.stackSmem));
     // deep stacks take the block past 48 KB of shared memory, which needs
     // the kernel's opt-in (a function attribute; harmless below that)
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
@@ -909,11 +846,11 @@ cudaError_t bh_launch_walk(const WalkArgs& in, bool fused, bool compensated, cud
     if (buckets && !a.nFirst) return cudaErrorInvalidValue;
     const int width = a.groupWidth ? a.groupWidth : 32;
     if (width != 32 && width != 64) return cudaErrorInvalidValue;
-    const bool wide = width == 64 && kWalkPacked;
+    const bool wide = width == 64;
     // one block per resident slot (the spill area is sized for bh_walk_grid(), the largest)
     const int maxBlocks = walk_min_blocks(a.relative, wide);
 #define BH_WALK_LAUNCH(F, C, R, B, W) \
-    return launch_walk_variant(k_walk<F, C, kWalkPacked, R, B, W && kWalkPacked>, a, maxBlocks, s)
+    return launch_walk_variant(k_walk<F, C, R, B, W>, a, maxBlocks, W, s)
 #define BH_WALK_BUCKETS(F, C, R)                                   \
     do {                                                           \
         if (wide) {                                                \
