@@ -7,7 +7,7 @@
 //   - one histogram read of the keys gives every digit's global counts
 //     (fused into the Morton kernel when the sort follows it);
 //   - one kernel per 8-bit digit: each CTA takes the next tile from an atomic
-//     counter, ranks its keys stably with warp ballots, publishes its
+//     counter, ranks its keys stably warp by warp, publishes its
 //     per-digit counts, and computes the count of each digit in all earlier
 //     tiles by decoupled look-back; it then scatters through shared memory so
 //     that each digit's run is written contiguously;
@@ -21,13 +21,10 @@
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-#ifndef BH_SORT_ITEMS
-#define BH_SORT_ITEMS 16
-#endif
-constexpr int kItems = BH_SORT_ITEMS;       // keys per thread
-constexpr int kTile = kThreads * kItems;    // 4096 keys per tile
+constexpr int kItems = 8;                 // keys per thread
+constexpr int kTile = kThreads * kItems;  // 4096 keys per tile
 constexpr uint32_t kFlagAgg = 1u << 30;     // tile count published
 constexpr uint32_t kFlagPrefix = 2u << 30;  // inclusive prefix published
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
@@ -86,50 +83,77 @@ __device__ __forceinline__ uint32_t lookback_exclusive(const uint32_t* status, i
 }  // namespace
 
 // Upfront digit histogram for a standalone sort: counts digits 0..npass-1 of
-// every key into hist[npass][256] (must be zero on entry).
-__global__ void __launch_bounds__(kThreads)
+// every key into hist[npass][256] (must be zero on entry).  Eight copies of
+// each bin in neighbouring banks (lane mod 8 takes its own), so that a warp
+// whose keys share a digit, as sorted or clustered keys do, waits four times
+// and not 32 times for one bin: 298 -> 60 us at 16.8M clustered
+// keys.
+constexpr int kHistCopies = 8;
+constexpr int kHistThreads = 512;
+__global__ void __launch_bounds__(kHistThreads)
 k_sort_histogram(const uint64_t* __restrict__ keys, int n, uint32_t* __restrict__ hist, int npass) {
-    __shared__ uint32_t sh[8][256];
-    for (int i = threadIdx.x; i < npass * 256; i += blockDim.x) (&sh[0][0])[i] = 0u;
+    extern __shared__ uint32_t sh[];  // [npass][256][kHistCopies]
+    const int bins = npass * 256;
+    for (int i = threadIdx.x; i < bins * kHistCopies; i += kHistThreads) sh[i] = 0u;
     __syncthreads();
-    const int per = 8;
-    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) * per; base < n;
-         base += gridDim.x * blockDim.x * per) {
-        const int cnt = (n - base < per) ? n - base : per;
+    const int stride = gridDim.x * kHistThreads;
+    uint32_t* mine = sh + (threadIdx.x & (kHistCopies - 1));
+    auto count = [&](uint64_t k) {
         for (int p = 0; p < npass; p++) {
-            uint32_t run = 0, cur = 0;
-            for (int j = 0; j < cnt; j++) {
-                const uint32_t d = (uint32_t)(__ldg(&keys[base + j]) >> (8 * p)) & 255u;
-                if (run && d != cur) { atomicAdd(&sh[p][cur], run); run = 0; }
-                cur = d;
-                run++;
-            }
-            if (run) atomicAdd(&sh[p][cur], run);
+            atomicAdd(mine + (p * 256 + (int)(k & 255u)) * kHistCopies, 1u);
+            k >>= 8;
         }
+    };
+    int i = blockIdx.x * kHistThreads + threadIdx.x;
+    for (; i + 3 * (long long)stride < n; i += 4 * stride) {  // four loads in flight
+        const uint64_t a = __ldg(&keys[i]), b = __ldg(&keys[i + stride]);
+        const uint64_t c = __ldg(&keys[i + 2 * stride]), d = __ldg(&keys[i + 3 * stride]);
+        count(a);
+        count(b);
+        count(c);
+        count(d);
     }
+    for (; i < n; i += stride) count(__ldg(&keys[i]));
     __syncthreads();
-    for (int i = threadIdx.x; i < npass * 256; i += blockDim.x) {
-        const uint32_t c = (&sh[0][0])[i];
-        if (c) atomicAdd(&hist[i], c);
+    for (int b = threadIdx.x; b < bins; b += kHistThreads) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < kHistCopies; k++) c += sh[b * kHistCopies + k];
+        if (c) atomicAdd(&hist[b], c);
     }
 }
 
 // One digit pass.  hist: the 256 global counts of this digit.  status:
 // [numTiles][256] words, zero on entry.  tileCounter: zero on entry.
 // identityVals: the values are the input positions (valsIn is not read).
-__global__ void __launch_bounds__(kThreads)
+//
+// A pass is bound by the chain of phases of one tile (loads, ranks, offsets,
+// look-back, scatter, stores) and then by shared-memory wavefronts (57% of
+// peak), not by HBM (0.45 of the copy rate at 16.8M), so a tile has many
+// threads with few keys each: 512 x 8 keys, two tiles per SM.  Ranks by a mask
+// per digit in shared memory instead of 8 ballots halve the instructions (194
+// -> 124 per 32 keys).  The second half of the threads looks back over the
+// earlier tiles while the first half already scatters, and the values are only
+// loaded for the scatter (registers).  Standalone sort of 63-bit keys at 16.8M
+// pairs 1638 -> 1152 us, 4.2M 464 -> 324, 1M 160 -> 110, 16,384 80 -> 57; the
+// step's sort stage at 1M 135 -> 105.  Measured and not kept: 3 tiles per SM
+// (40 registers, spills: 1234 us at 16.8M, 136 at 1M), 12 keys per thread
+// (1097 and 127), values loaded before the look-back (1160 and 111).
+__global__ void __launch_bounds__(kThreads, 2)
 k_sort_pass(const uint64_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
             uint64_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut, int n, int shift,
             const uint32_t* __restrict__ hist, uint32_t* status, int* tileCounter, int* err,
             int identityVals) {
     extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t* skeys = reinterpret_cast<uint64_t*>(smem);                        // kTile
-    uint32_t* svals = reinterpret_cast<uint32_t*>(skeys + kTile);               // kTile
-    uint32_t* warpHist = svals + kTile;                                         // [kWarps][256]
-    uint32_t* localStart = warpHist + kWarps * 256;                             // [256]
-    uint32_t* globalStart = localStart + 256;                                   // [256]
-    uint32_t* digitBase = globalStart + 256;                                    // [256]
+    uint64_t* skeys = reinterpret_cast<uint64_t*>(smem);           // kTile
+    uint32_t* svals = reinterpret_cast<uint32_t*>(skeys + kTile);  // kTile
+    uint32_t* warpHist = svals + kTile;                            // [kWarps][256]
+    uint32_t* warpMask = reinterpret_cast<uint32_t*>(smem);        // [kWarps][256]: lanes of a digit (before skeys is filled)
+    uint32_t* localStart = warpHist + kWarps * 256;                // [256]
+    uint32_t* tileCounts = localStart + 256;                       // [256]
+    uint32_t* target = tileCounts + 256;                           // [256]: output position of tile position 0
     __shared__ int sTile;
+    __shared__ uint32_t baseSum[8], countSum[8];
 
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     // programmatic dependent launch: the next pass may be scheduled once every
@@ -137,151 +161,160 @@ k_sort_pass(const uint64_t* __restrict__ keysIn, const uint32_t* __restrict__ va
     // upfront histograms) overlaps this pass's tail
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) sTile = atomicAdd(tileCounter, 1);
-    for (int i = tid; i < kWarps * 256; i += kThreads) warpHist[i] = 0u;
-    // exclusive scan of the global digit counts -> digit bases
-    {
-        const uint32_t c = hist[tid];
+    for (int i = tid; i < kWarps * 256; i += kThreads) {
+        warpHist[i] = 0u;
+        warpMask[i] = 0u;
+    }
+    // exclusive scan over one digit per thread (the first 256 threads), in
+    // two steps around a barrier
+    auto scanWarp = [&](uint32_t c, uint32_t* sums) {
         uint32_t x = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
-        if (lane == 31) localStart[w] = x;  // warp totals (temporary use)
-        __syncthreads();
-        uint32_t off = 0;
-        for (int k = 0; k < w; k++) off += localStart[k];
-        digitBase[tid] = off + x - c;
-    }
+        if (lane == 31) sums[w] = x;
+        return x - c;
+    };
+    auto scanBlock = [&](uint32_t x, const uint32_t* sums) {
+        for (int k = 0; k < w; k++) x += sums[k];
+        return x;
+    };
+    uint32_t digitBase = 0;  // first output position of digit tid
+    if (tid < 256) digitBase = scanWarp(hist[tid], baseSum);
     __syncthreads();
+    if (tid < 256) target[tid] = scanBlock(digitBase, baseSum);  // (read back by the thread that looks back)
     const int tile = sTile;
     const int tileBase = tile * kTile;
+    const int tileValid = n - tileBase < kTile ? n - tileBase : kTile;
     // the keys are the previous pass's output: wait for that grid to complete
     // (returns at once for a launch without a programmatic dependency)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // load: warp w owns keys [tileBase + w*32*kItems, +32*kItems), item k of
-    // lane l at offset k*32 + l (coalesced, and in input order k-major).
+    // lane l at offset k*32 + l (coalesced, and in input order k-major).  Past
+    // the end come keys of the highest digit: last in order, so they rank
+    // behind every key of the last tile and are never written out
     uint64_t key[kItems];
-    uint32_t val[kItems];
     uint32_t rank[kItems];
-    const int warpBase = tileBase + w * 32 * kItems;
+    const int warpOff = w * 32 * kItems + lane;
 #pragma unroll
     for (int k = 0; k < kItems; k++) {
-        const int i = warpBase + k * 32 + lane;
-        if (i < n) {
-            key[k] = keysIn[i];
-            val[k] = identityVals ? (uint32_t)i : valsIn[i];
-        } else {
-            key[k] = ~0ull;
-            val[k] = 0u;
-        }
+        const int i = warpOff + k * 32;
+        key[k] = i < tileValid ? keysIn[tileBase + i] : ~0ull;
     }
-    // stable ranks within the warp: items in order, peers by digit
+    auto digit = [&](int k) { return (uint32_t)(key[k] >> shift) & 255u; };
+    // stable ranks within the warp, items in order.  The lanes with the same
+    // digit meet in a mask per digit in shared memory (one atomic OR each);
+    // a warp whose keys all share the digit, as nearly sorted keys do in the
+    // high digits, is spared the 32 turns at one word
     uint32_t* myHist = warpHist + w * 256;
+    uint32_t* myMask = warpMask + w * 256;
+    const uint32_t lt = lanemask_lt();
 #pragma unroll
     for (int k = 0; k < kItems; k++) {
-        const int i = warpBase + k * 32 + lane;
-        const uint32_t valid = __ballot_sync(0xffffffffu, i < n);
-        const uint32_t d = (uint32_t)(key[k] >> shift) & 255u;
-        // lanes with the same digit: AND over the 8 digit bits of the ballot
-        // (or its complement) of that bit — 8 ballots, which measured 12-14%
-        // faster per sort than one __match_any_sync
-        uint32_t peers = valid;
-#pragma unroll
-        for (int bit = 0; bit < 8; bit++) {
-            const uint32_t m = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
-            peers &= ((d >> bit) & 1u) ? m : ~m;
+        const uint32_t d = digit(k);
+        uint32_t peers = 0xffffffffu, before;
+        if (__all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0))) {
+            before = myHist[d];
+            __syncwarp();
+            if (lane == 0) myHist[d] = before + 32u;
+        } else {
+            atomicOr(&myMask[d], 1u << lane);
+            __syncwarp();
+            peers = myMask[d];
+            before = myHist[d];
+            __syncwarp();
+            if ((peers & lt) == 0u) {  // the lowest peer moves the counter and clears the mask
+                myHist[d] = before + __popc(peers);
+                myMask[d] = 0u;
+            }
         }
-        uint32_t before = 0;
-        if (i < n) before = myHist[d];
-        __syncwarp();
-        if (i < n) {
-            rank[k] = before + __popc(peers & lanemask_lt());
-            if (lane == __ffs(peers) - 1) myHist[d] = before + __popc(peers);
-        }
+        rank[k] = before + __popc(peers & lt);
         __syncwarp();
     }
     __syncthreads();
-    // per digit: exclusive over warps, tile total
-    uint32_t tileCount;
-    {
-        const int d = tid;
-        uint32_t s = 0;
+    // per digit: tile total, published at once; then where each warp's keys of
+    // the digit start in the tile
+    uint32_t c[kWarps], start = 0, total = 0;
+    if (tid < 256) {
+#pragma unroll
+        for (int k = 0; k < kWarps; k++) c[k] = warpHist[k * 256 + tid];
+#pragma unroll
+        for (int k = 0; k < kWarps; k++) total += c[k];
+        st_volatile(status + (size_t)tile * 256 + tid, (tile == 0 ? kFlagPrefix : kFlagAgg) | total);
+        start = scanWarp(total, countSum);
+    }
+    __syncthreads();
+    if (tid < 256) {
+        start = scanBlock(start, countSum);
+        localStart[tid] = start;
+        tileCounts[tid] = total;
 #pragma unroll
         for (int k = 0; k < kWarps; k++) {
-            const uint32_t c = warpHist[k * 256 + d];
-            warpHist[k * 256 + d] = s;
-            s += c;
+            warpHist[k * 256 + tid] = start;
+            start += c[k];
         }
-        tileCount = s;
-        // publish, then look back over earlier tiles
-        uint32_t* myStatus = status + (size_t)tile * 256 + d;
-        if (tile == 0) {
-            st_volatile(myStatus, kFlagPrefix | s);
-            globalStart[d] = digitBase[d];
-        } else {
-            st_volatile(myStatus, kFlagAgg | s);
-            const uint32_t excl = lookback_exclusive(status, tile, d, err);
-            st_volatile(myStatus, kFlagPrefix | ((excl + s) & kValueMask));
-            globalStart[d] = digitBase[d] + excl;
-        }
-    }
-    // tile-local start of each digit (exclusive scan of tileCount over digits)
-    {
-        uint32_t x = tileCount;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        __shared__ uint32_t wsum[kWarps];
-        if (lane == 31) wsum[w] = x;
-        __syncthreads();
-        uint32_t off = 0;
-        for (int k = 0; k < w; k++) off += wsum[k];
-        localStart[tid] = off + x - tileCount;
     }
     __syncthreads();
+    if (tid >= 256) {  // look back over earlier tiles
+        const int d = tid - 256;
+        uint32_t excl = 0;
+        if (tile > 0) {
+            excl = lookback_exclusive(status, tile, d, err);
+            st_volatile(status + (size_t)tile * 256 + d, kFlagPrefix | ((excl + tileCounts[d]) & kValueMask));
+        }
+        target[d] += excl - localStart[d];
+    }
     // scatter into shared memory in sorted-within-tile order
+    uint32_t val[kItems];
 #pragma unroll
     for (int k = 0; k < kItems; k++) {
-        const int i = warpBase + k * 32 + lane;
-        if (i < n) {
-            const uint32_t d = (uint32_t)(key[k] >> shift) & 255u;
-            const uint32_t p = localStart[d] + warpHist[w * 256 + d] + rank[k];
-            skeys[p] = key[k];
-            svals[p] = val[k];
-        }
+        const int i = warpOff + k * 32;
+        val[k] = 0u;
+        if (i < tileValid) val[k] = identityVals ? (uint32_t)(tileBase + i) : valsIn[tileBase + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; k++) {
+        const uint32_t p = myHist[digit(k)] + rank[k];
+        skeys[p] = key[k];
+        svals[p] = val[k];
     }
     __syncthreads();
     // write out: consecutive positions of a digit go to consecutive addresses
-    const int tileValid = (n - tileBase < kTile) ? n - tileBase : kTile;
-    for (int j = tid; j < tileValid; j += kThreads) {
-        const uint64_t k = skeys[j];
-        const uint32_t d = (uint32_t)(k >> shift) & 255u;
-        const uint32_t dst = globalStart[d] + (uint32_t)j - localStart[d];
-        keysOut[dst] = k;
-        valsOut[dst] = svals[j];
+#pragma unroll
+    for (int k = 0; k < kItems; k++) {
+        const int j = tid + k * kThreads;
+        if (j < tileValid) {
+            const uint64_t q = skeys[j];
+            const uint32_t dst = target[(uint32_t)(q >> shift) & 255u] + (uint32_t)j;
+            keysOut[dst] = q;
+            valsOut[dst] = svals[j];
+        }
     }
 }
 
 // ---------------------------------------------------------------- launchers
 namespace {
 size_t pass_smem() { return (size_t)kTile * (8 + 4) + (size_t)(kWarps * 256 + 3 * 256) * 4; }
+size_t hist_smem(int npass) { return (size_t)npass * 256 * kHistCopies * 4; }
 }  // namespace
 
 int bh_sort_tile() { return kTile; }
 
 cudaError_t bh_sort_init() {
-    return cudaFuncSetAttribute(k_sort_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem());
+    const cudaError_t e = cudaFuncSetAttribute(k_sort_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem());
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k_sort_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)hist_smem(8));
 }
 
 cudaError_t bh_launch_sort_histogram(const uint64_t* keys, int n, uint32_t* hist, int npass, cudaStream_t s) {
-    int grid = (n + kThreads * 8 - 1) / (kThreads * 8);
-    const int cap = 4 * bh_sm_count();
+    int grid = (n + kHistThreads * 8 - 1) / (kHistThreads * 8);
+    const int cap = 3 * bh_sm_count();  // resident at once with 64 KB of counters each
     grid = grid < 1 ? 1 : (grid > cap ? cap : grid);
-    k_sort_histogram<<<grid, kThreads, 0, s>>>(keys, n, hist, npass);
+    k_sort_histogram<<<grid, kHistThreads, hist_smem(npass), s>>>(keys, n, hist, npass);
     return cudaGetLastError();
 }
 
