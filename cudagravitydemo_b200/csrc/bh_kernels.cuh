@@ -32,6 +32,12 @@ cudaError_t bh_sort_init();  // raises the dynamic shared-memory limit once
 // (status[0..511] must be zero): gives up after BH_SPIN_LIMIT round trips and
 // sets BH_ERR_TIMEOUT in *err.  Exercises the bounded wait without a fault.
 cudaError_t bh_launch_lookback_selftest(const uint32_t* status, int* err, cudaStream_t s);
+// A whole stable sort by the low 8 * npass bits in one launch, for at most
+// bh_sort_cluster_limit() pairs; valsIn NULL: the values are the input
+// positions.  Needs no scratch.
+int bh_sort_cluster_limit();
+cudaError_t bh_launch_sort_cluster(const uint64_t* keysIn, const uint32_t* valsIn, uint64_t* keysOut, uint32_t* valsOut,
+                                   int n, int npass, cudaStream_t s);
 cudaError_t bh_launch_sort_histogram(const uint64_t* keys, int n, uint32_t* hist, int npass, cudaStream_t s);
 cudaError_t bh_launch_sort_pass(const uint64_t* keysIn, const uint32_t* valsIn, uint64_t* keysOut,
                                 uint32_t* valsOut, int n, int shift, const uint32_t* hist,

@@ -7,7 +7,7 @@
 // kernels with no host synchronisation inside:
 //   k_bbox (world box on the device, histograms zeroed)
 //   k_morton (keys + radix digit histograms)
-//   k_sort_pass x ceil(3*bits/8)
+//   k_sort_pass x ceil(3*bits/8), or k_sort_cluster for small n
 //   k_reorder (pos, vel, body ids)
 //   k_tree_count, k_tree_scan, k_tree_nodes, k_tree_mass [, k_tree_export]
 //   k_walk (+ fused kick-drift)
@@ -244,12 +244,22 @@ static bh_ctx* ctx_of(const treeState* st) {
     return c->magic == kCtxMagic ? c : nullptr;
 }
 
+// Where the keys kernel counts the digits of n keys for the sort that follows
+// (NULL when that sort, in one cluster, wants no counts).
+static uint32_t* ctx_sort_histogram(const bh_ctx* c, int n) {
+    return n <= bh_sort_cluster_limit() ? nullptr : c->sortHist;
+}
+
 // Stable sort of n pairs by the low keyBits bits.  valsIn == NULL: values are
 // the input positions.  histReady: sortHist already holds this input's digit
 // counts (the keys kernel produced them).
 static int ctx_sort(bh_ctx* c, const uint64_t* keysIn, const uint32_t* valsIn, uint64_t* keysOut,
                     uint32_t* valsOut, int n, int keyBits, bool histReady, cudaStream_t s) {
     const int npass = (keyBits + 7) / 8;
+    if (n <= bh_sort_cluster_limit()) {
+        BH_CUDA_TRY(bh_launch_sort_cluster(keysIn, valsIn, keysOut, valsOut, n, npass, s));
+        return BH_OK;
+    }
     const int tiles = (n + bh_sort_tile() - 1) / bh_sort_tile();
     BH_CUDA_TRY(cudaMemsetAsync(c->sortStatus, 0, sizeof(uint32_t) * (256 + (size_t)npass * tiles * 256), s));
     if (!histReady) {
@@ -394,12 +404,13 @@ extern "C" int bh_build_tree(treeState* st, float4** pos, float3** vel, cudaStre
     } while (0)
 #define TRYC(x) TRY(((x) == cudaSuccess) ? BH_OK : bh_note_cuda_error(cudaGetLastError()))
     TRY(cudaMemsetAsync(c->err, 0, sizeof(int), s) == cudaSuccess ? BH_OK : BH_ERR_CUDA);
+    uint32_t* const hist = ctx_sort_histogram(c, n);
     // stage 1: world box (basicGravity.cu:143-155)
     TRYC(bh_launch_bbox(*pos, n, c->bboxPartials, c->bboxTicket, c->box, st->boundingData[2], st->boundingData[3],
-                        bits, c->err, c->sortHist, 8 * 256, s, c->bboxPartials64, c->root64));
+                        bits, c->err, hist, hist ? 8 * 256 : 0, s, c->bboxPartials64, c->root64));
     // stage 2: keys (basicGravity.cu:176-183)
     worldBox none = {0, 0, 0, 0, 0};
-    TRYC(bh_launch_morton(*pos, n, c->box, none, bits, st->mortonIn, st->indexIn, c->sortHist, 8, s));
+    TRYC(bh_launch_morton(*pos, n, c->box, none, bits, st->mortonIn, st->indexIn, hist, 8, s));
     // stage 3: sort + reorder + pointer swap (basicGravity.cu:190-226)
     TRY(ctx_sort(c, st->mortonIn, st->indexIn, st->mortonOut, st->indexOut, n, 64, true, s));
     TRYC(bh_launch_reorder(*pos, *vel, nullptr, st->indexOut, st->sortedPosMassVals, st->sortedVelVals, nullptr,
@@ -1075,17 +1086,17 @@ static int sim_enqueue_build(bh_sim* s, cudaEvent_t* ev, cudaEvent_t afterReorde
     const int keyBits = 3 * bits + (s->systems ? s->sysBits : 0);
     const int npass = (keyBits + 7) / 8;
     cudaStream_t st = s->stream;
+    uint32_t* const hist = ctx_sort_histogram(c, n);
+    const int histWords = hist ? npass * 256 : 0;
     if (ev) BH_CUDA_TRY(cudaEventRecord(ev[0], st));
     worldBox none = {0, 0, 0, 0, 0};
     if (s->systems) {
-        BH_CUDA_TRY(bh_launch_bbox_segments(s->posA, s->segOff, s->systems, s->boxes, bits, c->err, c->sortHist,
-                                            npass * 256, st));
-        BH_CUDA_TRY(bh_launch_morton(s->posA, n, s->boxes, none, bits, s->keysA, nullptr, c->sortHist, npass, st,
-                                     s->sysOf));
+        BH_CUDA_TRY(bh_launch_bbox_segments(s->posA, s->segOff, s->systems, s->boxes, bits, c->err, hist, histWords, st));
+        BH_CUDA_TRY(bh_launch_morton(s->posA, n, s->boxes, none, bits, s->keysA, nullptr, hist, npass, st, s->sysOf));
     } else {
         BH_CUDA_TRY(bh_launch_bbox(s->posA, n, c->bboxPartials, c->bboxTicket, c->box, s->corner, s->corner + 1,
-                                   bits, c->err, c->sortHist, npass * 256, st, c->bboxPartials64, c->root64));
-        BH_CUDA_TRY(bh_launch_morton(s->posA, n, c->box, none, bits, s->keysA, nullptr, c->sortHist, npass, st));
+                                   bits, c->err, hist, histWords, st, c->bboxPartials64, c->root64));
+        BH_CUDA_TRY(bh_launch_morton(s->posA, n, c->box, none, bits, s->keysA, nullptr, hist, npass, st));
     }
     if (ev) BH_CUDA_TRY(cudaEventRecord(ev[1], st));
     int rc = ctx_sort(c, s->keysA, nullptr, s->keysB, s->perm, n, keyBits, true, st);
@@ -1226,8 +1237,9 @@ static int sim_enqueue_step(bh_sim* s, cudaEvent_t* ev) {
 // Kernel launches of one step (the count the benchmark reports).
 extern "C" int bh_sim_kernels_per_step(const bh_sim* s) {
     if (!s) return 0;
-    const int npass = (3 * sim_bits(s) + (s->systems ? s->sysBits : 0) + 7) / 8;
-    return 2 /* box, keys */ + npass + 1 /* reorder */ + 4 /* tree */ + (s->prm.exportNodes ? 1 : 0) +
+    const int digits = (3 * sim_bits(s) + (s->systems ? s->sysBits : 0) + 7) / 8;
+    const int npass = (s->n > 0 ? s->n : s->capacity) <= bh_sort_cluster_limit() ? 1 : digits;
+    return 2 /* box, keys */ + npass /* sort */ + 1 /* reorder */ + 4 /* tree */ + (s->prm.exportNodes ? 1 : 0) +
            (s->prm.macMode == 2 ? 2 : 0) /* features, selection */ + 2 /* group order */ + 1 /* walk */;
 }
 

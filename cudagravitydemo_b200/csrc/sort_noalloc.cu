@@ -100,6 +100,11 @@ int sort_noalloc(const uint64_t* keysIn, uint64_t* keysOut, const uint32_t* vals
     int* err = reinterpret_cast<int*>(base + kErrOff);
 
     const int npass = (keyBits + 7) / 8;
+    if (n <= bh_sort_cluster_limit()) {  // needs nothing of the scratch but the error word, which it leaves clear
+        BH_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), s));
+        BH_CUDA_TRY(bh_launch_sort_cluster(keysIn, valsIn, keysOut, valsOut, n, npass, s));
+        return BH_OK;
+    }
     const int tiles = (n + kSortTile - 1) / kSortTile;
     // what must start at zero: histograms, tile counters, look-back words,
     // the error word (a previous call leaves them dirty)

@@ -1,5 +1,6 @@
-"""The radix sort at the edges of its tiles (4,096 pairs, 32 per warp and item)
-and with digits that a warp shares wholly, partly or not at all."""
+"""The radix sort at the edges of its tiles (4,096 pairs, 32 per warp and item),
+of its one-cluster form (1,024 pairs per block, 16 blocks, one or two keys per
+thread) and with digits that a warp shares wholly, partly or not at all."""
 from __future__ import annotations
 
 import ctypes
@@ -9,7 +10,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 31, 33, 255, 256, 257, 4095, 4096, 4097, 8191, 8193, 12288, 40961, 300007]
+SIZES = [1, 2, 31, 33, 255, 256, 257, 1023, 1024, 1025, 4095, 4097, 16383, 16384, 16385, 18433, 32767, 32768, 32769,
+         36864, 40961, 300007]
 
 
 def _keys(rng, n, kind):
