@@ -63,9 +63,8 @@ cudaError_t bh_launch_tree_mass(const float4* pos, const uint8_t* delta, int n, 
                                 const int2* nCB, float4* nCom, WalkNode* wn, const int* nFirst, int* nCount,
                                 unsigned* bar, int* err, cudaStream_t s);
 cudaError_t bh_launch_tree_export(const uint64_t* keys, int bits, const DevTreeInfo* info,
-                                  const WalkNode* wn, const int* nParent, const int* nFirst,
-                                  const int* nCount, const int* nMeta, node* out, int n, int maxNodes,
-                                  cudaStream_t s);
+                                  const WalkNode* wn, const int* nParent, const int* nFirst, const int* nMeta, node* out,
+                                  int n, int maxNodes, cudaStream_t s);
 // auxIn/auxOut: an optional per-body float carried along (NULL: none)
 cudaError_t bh_launch_reorder(const float4* posIn, const float3* velIn, const uint32_t* idIn,
                               const uint32_t* perm, float4* posOut, float3* velOut, uint32_t* idOut,

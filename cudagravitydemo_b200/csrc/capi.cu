@@ -306,8 +306,8 @@ static int ctx_build(bh_ctx* c, const uint64_t* sortedKeys, const float4* sorted
                                     c->nCount, c->gridBar, c->err, s));
     if (ev) BH_CUDA_TRY(cudaEventRecord(ev[3], s));
     if (exportTo)
-        BH_CUDA_TRY(bh_launch_tree_export(sortedKeys, bits, c->info, c->wn, c->nParent, c->nFirst, c->nCount,
-                                          c->nMeta, exportTo, n, c->maxNodes, s));
+        BH_CUDA_TRY(bh_launch_tree_export(sortedKeys, bits, c->info, c->wn, c->nParent, c->nFirst, c->nMeta, exportTo, n,
+                                          c->maxNodes, s));
     return BH_OK;
 }
 

@@ -160,31 +160,35 @@ k_tree_scan(int* __restrict__ blockLevel, int nblocks, int n, int bits, int maxN
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || tid != 0) return;
+    if (!last || w != 0) return;
+    // one level per lane (in one thread, level after level, it took a third of
+    // the kernel's own time: 10.4 -> 8.6 us between events at 1,000 bodies)
     __threadfence();
-    DevTreeInfo t;
-    int off = 0, deepest = 0, overflow = 0;
-    for (int k = 0; k < BH_LEVEL_SLOTS; k++) {
-        const int c = (k <= bits) ? __ldcg(&levelTotal[k]) : 0;
-        t.levelOffset[k] = off;
-        t.levelCount[k] = c;
-        if (c > 0) deepest = k;
-        if (!overflow && c > 0 && off + c > maxNodes) overflow = k;
-        off += c;
+    const int c = lane <= bits ? __ldcg(&levelTotal[lane]) : 0;
+    int after = c;  // nodes up to and including this level
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, after, o);
+        if (lane >= o) after += y;
     }
-    t.deepest = deepest;
-    t.nodeCount = off;
-    t.overflowLevel = overflow;
-    t.pad = 0;
-    const float extX = box->extX;  // the first system's (the only one outside a batch)
-    for (int k = 0; k < BH_LEVEL_SLOTS; k++) {
-        const float sz = ldexpf(extX, -k);  // exact: extX / 2^k
-        t.sizeSq[k] = __fmul_rn(sz, sz);
+    const int nodes = __shfl_sync(0xffffffffu, after, 31);
+    const unsigned used = __ballot_sync(0xffffffffu, c > 0), over = __ballot_sync(0xffffffffu, c > 0 && after > maxNodes);
+    const int overflow = over ? __ffs(over) - 1 : 0;
+    if (lane < BH_LEVEL_SLOTS) {
+        info->levelOffset[lane] = after - c;
+        info->levelCount[lane] = c;
+        const float sz = ldexpf(box->extX, -lane);  // exact: extX / 2^level; the first system's (the only one outside a batch)
+        info->sizeSq[lane] = __fmul_rn(sz, sz);
     }
-    *info = t;
-    if (overflow) bh_set_error(err, BH_ERR_TREE_OVERFLOW);
-    else nCB[off].x = off;  // sentinel: end of the last child range
-    *ticket = 0u;           // re-armed for the next build
+    if (lane == 0) {
+        info->deepest = used ? 31 - __clz(used) : 0;
+        info->nodeCount = nodes;
+        info->overflowLevel = overflow;
+        info->pad = 0;
+        if (overflow) bh_set_error(err, BH_ERR_TREE_OVERFLOW);
+        else nCB[nodes].x = nodes;  // sentinel: end of the last child range
+        *ticket = 0u;               // re-armed for the next build
+    }
 }
 
 // Pass 3: node records.  For body i with node range [lo, hi] and level-L
@@ -318,6 +322,59 @@ __device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned target, int
 }
 
 
+// A leaf's centre of mass, mass and count of bodies: node k of level L, no children.
+__device__ __forceinline__ float4 leaf_mass(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, int n,
+                                            int bits, const int* __restrict__ nFirst, int nodeCount, int k, int L,
+                                            int& count) {
+    const int first = (k == 0) ? 0 : nFirst[k];
+    if (nodeCount == 1) {
+        count = n;
+    } else if (L == bits) {
+        int j = first + 1;
+        while (j < n && (int)delta[j] == bits) j++;
+        count = j - first;
+    } else {
+        count = 1;
+    }
+    float wx = 0.f, wy = 0.f, wz = 0.f, m = 0.f;
+    for (int t = 0; t < count; t++) {
+        const float4 p = pos[first + t];
+        wx = __fmaf_rn(p.x, p.w, wx);
+        wy = __fmaf_rn(p.y, p.w, wy);
+        wz = __fmaf_rn(p.z, p.w, wz);
+        m = __fadd_rn(m, p.w);
+    }
+    return m > 0.0f ? make_float4(__fdiv_rn(wx, m), __fdiv_rn(wy, m), __fdiv_rn(wz, m), m)
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// The same of an internal node from its nch children (at most 8).
+__device__ __forceinline__ float4 children_mass(const float4 cm[8], const int cc[8], int nch, int& count) {
+    float m = 0.f, x = 0.f, y = 0.f, z = 0.f;
+    count = 0;
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+        if (t < nch) {
+            m = __fadd_rn(m, cm[t].w);
+            count += cc[t];
+        }
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+        if (t < nch) {
+            x = __fmaf_rn(cm[t].x, cm[t].w, x);
+            y = __fmaf_rn(cm[t].y, cm[t].w, y);
+            z = __fmaf_rn(cm[t].z, cm[t].w, z);
+        }
+    return m > 0.0f ? make_float4(__fdiv_rn(x, m), __fdiv_rn(y, m), __fdiv_rn(z, m), m) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// The walk's record in one 32-byte store pair.
+__device__ __forceinline__ void put_record(WalkNode* wn, int k, float4 com, int cb, int ce, int sizeBits, int count) {
+    float4* rec = reinterpret_cast<float4*>(&wn[k]);
+    rec[0] = com;
+    rec[1] = make_float4(__int_as_float(cb), __int_as_float(ce), __int_as_float(sizeBits), __int_as_float(count));
+}
+
 __global__ void __launch_bounds__(kMassThreads)
 k_tree_mass(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, int n, int bits,
             const DevTreeInfo* __restrict__ info, const int2* __restrict__ nCB, float4* nCom, WalkNode* __restrict__ wn,
@@ -340,28 +397,10 @@ k_tree_mass(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, i
             const int2 me = nCB[k];
             const int cb = me.x;
             const int ce = nCB[k + 1].x;
-            float4 com = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 com;
             int count;
-            if (cb == ce) {  // leaf
-                const int first = (k == 0) ? 0 : nFirst[k];
-                if (nodeCount == 1) {
-                    count = n;
-                } else if (L == bits) {
-                    int j = first + 1;
-                    while (j < n && (int)delta[j] == bits) j++;
-                    count = j - first;
-                } else {
-                    count = 1;
-                }
-                float wx = 0.f, wy = 0.f, wz = 0.f, m = 0.f;
-                for (int t = 0; t < count; t++) {
-                    const float4 p = pos[first + t];
-                    wx = __fmaf_rn(p.x, p.w, wx);
-                    wy = __fmaf_rn(p.y, p.w, wy);
-                    wz = __fmaf_rn(p.z, p.w, wz);
-                    m = __fadd_rn(m, p.w);
-                }
-                if (m > 0.0f) com = make_float4(__fdiv_rn(wx, m), __fdiv_rn(wy, m), __fdiv_rn(wz, m), m);
+            if (cb == ce) {
+                com = leaf_mass(pos, delta, n, bits, nFirst, nodeCount, k, L, count);
             } else {
                 const int nch = ce - cb;
                 if (nch > 8 || cb <= k) {  // broken links: report, do not follow
@@ -377,28 +416,10 @@ k_tree_mass(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, i
                         cc[t] = __ldcg(&nCount[cb + t]);
                     }
                 }
-                float m = 0.f, x = 0.f, y = 0.f, z = 0.f;
-                count = 0;
-#pragma unroll
-                for (int t = 0; t < 8; t++)
-                    if (t < nch) {
-                        m = __fadd_rn(m, cm[t].w);
-                        count += cc[t];
-                    }
-#pragma unroll
-                for (int t = 0; t < 8; t++)
-                    if (t < nch) {
-                        x = __fmaf_rn(cm[t].x, cm[t].w, x);
-                        y = __fmaf_rn(cm[t].y, cm[t].w, y);
-                        z = __fmaf_rn(cm[t].z, cm[t].w, z);
-                    }
-                if (m > 0.0f) com = make_float4(__fdiv_rn(x, m), __fdiv_rn(y, m), __fdiv_rn(z, m), m);
+                com = children_mass(cm, cc, nch, count);
             }
-            // the walk's record in one 32-byte store pair; the compact copies
-            // serve the parent level
-            float4* rec = reinterpret_cast<float4*>(&wn[k]);
-            rec[0] = com;
-            rec[1] = make_float4(__int_as_float(cb), __int_as_float(ce), __int_as_float(me.y), __int_as_float(count));
+            // the compact copies serve the parent level
+            put_record(wn, k, com, cb, ce, me.y, count);
             nCom[k] = com;
             nCount[k] = count;
         }
@@ -413,13 +434,86 @@ k_tree_mass(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, i
     }
 }
 
+// The upward pass of a small tree by one block: all nodes' child ranges and the
+// leaves first, side by side, then the levels from shared memory, where a level
+// costs a block barrier instead of a grid barrier and three round trips to L2.
+// Between events: 1,000 bodies 27.0 -> 16.5 us, 4,000 36 -> 26.  (A tree of more nodes than the shared
+// memory holds, long chains of single children, reads the compact copies.)
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallNodes = 8000;   // 28 bytes each
+constexpr int kSmallBodies = 4096;  // 1.5 nodes per body as a rule
+constexpr size_t kSmallMem = (size_t)kSmallNodes * 28 + 16;
+__global__ void __launch_bounds__(kSmallThreads)
+k_tree_mass_small(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, int n, int bits,
+                  const DevTreeInfo* __restrict__ info, const int2* __restrict__ nCB, float4* nCom,
+                  WalkNode* __restrict__ wn, const int* __restrict__ nFirst, int* nCount, int* err) {
+    extern __shared__ __align__(16) float4 sCom[];
+    int* const sCount = reinterpret_cast<int*>(sCom + kSmallNodes);
+    int* const sSize = sCount + kSmallNodes;
+    int* const sFirst = sSize + kSmallNodes;  // first child
+    if (info->overflowLevel) return;
+    const int nodeCount = info->nodeCount;
+    const bool held = nodeCount < kSmallNodes;
+    for (int k = threadIdx.x; k < nodeCount; k += kSmallThreads) {
+        const int2 me = nCB[k];
+        const int cb = me.x, ce = nCB[k + 1].x;
+        float4 com = make_float4(0.f, 0.f, 0.f, 0.f);
+        int count = 0;
+        if (cb == ce) {
+            const int L = k >= info->levelOffset[bits] ? bits : 0;  // (which other level does not matter)
+            com = leaf_mass(pos, delta, n, bits, nFirst, nodeCount, k, L, count);
+            put_record(wn, k, com, cb, ce, me.y, count);
+        }
+        if (held) {
+            sCom[k] = com;
+            sCount[k] = count;
+            sSize[k] = me.y;
+            sFirst[k] = cb;
+            if (k == nodeCount - 1) sFirst[nodeCount] = ce;
+        } else {
+            nCom[k] = com;
+            nCount[k] = count;
+        }
+    }
+    __syncthreads();
+    for (int L = info->deepest; L >= 0; L--) {
+        const int begin = info->levelOffset[L], end = begin + info->levelCount[L];
+        for (int k = begin + threadIdx.x; k < end; k += kSmallThreads) {
+            const int cb = held ? sFirst[k] : nCB[k].x, ce = held ? sFirst[k + 1] : nCB[k + 1].x, nch = ce - cb;
+            if (nch == 0) continue;
+            if (nch < 0 || nch > 8 || cb <= k) {  // broken links: report, do not follow
+                bh_set_error(err, BH_ERR_INTERNAL);
+                continue;
+            }
+            float4 cm[8];
+            int cc[8];
+#pragma unroll
+            for (int t = 0; t < 8; t++)
+                if (t < nch) {
+                    cm[t] = held ? sCom[cb + t] : __ldcg(&nCom[cb + t]);
+                    cc[t] = held ? sCount[cb + t] : __ldcg(&nCount[cb + t]);
+                }
+            int count;
+            const float4 com = children_mass(cm, cc, nch, count);
+            put_record(wn, k, com, cb, ce, held ? sSize[k] : nCB[k].y, count);
+            if (held) {
+                sCom[k] = com;
+                sCount[k] = count;
+            } else {
+                nCom[k] = com;
+                nCount[k] = count;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // Reference layout (types.h:52-62): one thread per node writes the 80-byte
 // record, child[slot] from the contiguous child range.
 __global__ void __launch_bounds__(256)
 k_tree_export(const uint64_t* __restrict__ keys, int bits, const DevTreeInfo* __restrict__ info,
               const WalkNode* __restrict__ wn, const int* __restrict__ nParent,
-              const int* __restrict__ nFirst, const int* __restrict__ nCount,
-              const int* __restrict__ nMeta, node* __restrict__ out, int n) {
+              const int* __restrict__ nFirst, const int* __restrict__ nMeta, node* __restrict__ out, int n) {
     if (info->overflowLevel) return;
     const int nodeCount = info->nodeCount;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nodeCount; k += gridDim.x * blockDim.x) {
@@ -430,7 +524,7 @@ k_tree_export(const uint64_t* __restrict__ keys, int bits, const DevTreeInfo* __
         r.nodePathFromRoot = (k == 0) ? 0ull : level_prefix(keys[first], bits, level);
         r.parentIndex = (k == 0) ? -1 : nParent[k];
         r.firstParticleIndex = first;
-        r.particleCount = (k == 0) ? n : nCount[k];
+        r.particleCount = (k == 0) ? n : w.count;
 #pragma unroll
         for (int s = 0; s < 8; s++) r.child[s] = -1;
         const int ce = w.childEnd < w.childBegin + 8 ? w.childEnd : w.childBegin + 8;
@@ -556,10 +650,20 @@ int bh_tree_mass_grid() {
 cudaError_t bh_launch_tree_mass(const float4* pos, const uint8_t* delta, int n, int bits, const DevTreeInfo* info,
                                 const int2* nCB, float4* nCom, WalkNode* wn, const int* nFirst, int* nCount,
                                 unsigned* bar, int* err, cudaStream_t s) {
+    if (n <= kSmallBodies) {
+        const cudaError_t e = cudaFuncSetAttribute(k_tree_mass_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)kSmallMem);
+        if (e != cudaSuccess) return e;
+        k_tree_mass_small<<<1, kSmallThreads, kSmallMem, s>>>(pos, delta, n, bits, info, nCB, nCom, wn, nFirst, nCount,
+                                                              err);
+        return cudaGetLastError();
+    }
     cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(bh_tree_mass_grid());
+    // (a level has at most one node per body)
+    const int most = (n + kMassThreads - 1) / kMassThreads, all = bh_tree_mass_grid();
+    cfg.gridDim = dim3(most < all ? most : all);
     cfg.blockDim = dim3(kMassThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
@@ -572,11 +676,9 @@ cudaError_t bh_launch_tree_mass(const float4* pos, const uint8_t* delta, int n, 
 }
 
 cudaError_t bh_launch_tree_export(const uint64_t* keys, int bits, const DevTreeInfo* info,
-                                  const WalkNode* wn, const int* nParent, const int* nFirst,
-                                  const int* nCount, const int* nMeta, node* out, int n, int maxNodes,
-                                  cudaStream_t s) {
-    k_tree_export<<<stream_grid(maxNodes, 256), 256, 0, s>>>(keys, bits, info, wn, nParent, nFirst, nCount, nMeta,
-                                                               out, n);
+                                  const WalkNode* wn, const int* nParent, const int* nFirst, const int* nMeta, node* out,
+                                  int n, int maxNodes, cudaStream_t s) {
+    k_tree_export<<<stream_grid(maxNodes, 256), 256, 0, s>>>(keys, bits, info, wn, nParent, nFirst, nMeta, out, n);
     return cudaGetLastError();
 }
 
