@@ -830,14 +830,23 @@ static cudaError_t launch_walk_variant(Kernel kernel, const WalkArgs& a, int max
     if (e != cudaSuccess) return e;
     resident = resident < maxBlocks ? resident : maxBlocks;
     if (resident < 1) return cudaErrorInvalidConfiguration;
-    // a walk of few groups launches no warps that would only find the cursor
-    // at its end, and its blocks spread over the SMs (512 groups taken by the
-    // first warps of a full grid sat on few SMs: 155 us at 16,384 bodies, 93
-    // with a grid of their own)
-    const int perGroup = wide ? 64 : 32;
-    const int groups = a.groupTable ? a.groups : (a.n + perGroup - 1) / perGroup;
-    const int all = bh_sm_count() * resident, some = (groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    kernel<<<some < all ? some : all, kThreads, dyn, s>>>(a);
+    // How many warps share the groups.  A walk of few groups launches no warps
+    // that would only find the cursor at its end, and its blocks spread over the
+    // SMs (512 groups taken by the first warps of a full grid sat on few SMs: 155
+    // us at 16,384 bodies, 93 with a grid of their own).  Up to ten groups per
+    // sub-partition, half of them plus one are walked at once: the groups come
+    // longest first, so a warp that is done takes a short one, and fewer at once
+    // leave no half-empty last wave (walk of theta 0.5 disks / Plummer spheres, us
+    // with six warps per sub-partition and with this many: 60,000 bodies 146 / 168
+    // and 143 / 167, 80,000 180 / 199 and 165 / 180, 100,000 206 / 211 and 173 / 195,
+    // 150,000 235 / 250 and 220 / 244; half of them without the one more: 134 / 200
+    // at 60,000, Plummer spheres have a few long groups).
+    const int perGroup = wide ? 64 : 32, sms = bh_sm_count();
+    const long long groups = a.groupTable ? a.groups : (a.n + perGroup - 1) / perGroup;
+    const long long half = (groups - 1) / (2ll * kWarpsPerBlock * sms) + 1;  // rounded up
+    const int perSm = half + 1 < resident ? (int)half + 1 : resident;
+    const long long all = (long long)sms * perSm, some = (groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    kernel<<<(unsigned)(some < all ? some : all), kThreads, dyn, s>>>(a);
     return cudaGetLastError();
 }
 
