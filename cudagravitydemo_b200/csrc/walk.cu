@@ -89,8 +89,23 @@ constexpr int kMinBlocksRelative = BH_WALK_MIN_BLOCKS_RELATIVE;
 // 64-body groups (two bodies per lane), every criterion: 4 blocks (up to 128
 // registers; 110 used) measured 7% faster than 6 blocks with spills
 constexpr int kMinBlocksWide = BH_WALK_MIN_BLOCKS_WIDE;
-__host__ __device__ constexpr int walk_min_blocks(bool relative, bool wide) {
-    return wide ? kMinBlocksWide : (relative ? kMinBlocksRelative : kMinBlocksPlain);
+// Few 32-body groups: the time is one long group's chain of rounds, and warps in
+// other slots hide nothing.  More registers (3 blocks, up to 168; 138 to 150 used)
+// let one warp overlap its own entries: a list of 224 takes 3,650 cycles instead
+// of 7,550 (the FMA pipe alone needs 3,600), a vote unrolled whole 1,120 instead of
+// 1,500.  Walk before and after, us, theta 0.5 Plummer spheres unless said: 1,000
+// bodies 42 and 39, 4,000 76 and 66, 16,384 92 and 80, 36,000 145 and 133, 60,000
+// 170 and 164, 100,000 203 and 195; disks of 80,000 171 and 145, learned of 100,000
+// 203 and 183.  Beyond that throughput counts again: 125,000 225 and 232 (a disk 211
+// and 199), 150,000 254 and 268, 262,144 learned 416 and 444.  The line is drawn
+// at 24 groups per SM (113,000 bodies).  Blocks of 2 and 4 per SM were the same up
+// to 36,000 bodies, 226 and 187 us at 100,000, 151 and 169 at the disk of 80,000;
+// prefetching the children of opened nodes into L1 gave nothing (80 to 82 us at
+// 16,384), and evaluators in warps of their own beside the walker gave less (82).
+constexpr int kMinBlocksFew = 3;
+constexpr int kFewGroupsPerSm = 24;
+__host__ __device__ constexpr int walk_min_blocks(bool relative, bool wide, bool few) {
+    return few ? kMinBlocksFew : wide ? kMinBlocksWide : (relative ? kMinBlocksRelative : kMinBlocksPlain);
 }
 constexpr int kBlocksPerSm = 8;  // persistent grid: blocks launched per SM (the excess waits)
 constexpr int kSpillPerWarp = 4096;  // global stack entries per warp beyond shared memory
@@ -207,9 +222,10 @@ __device__ __forceinline__ float ref_dist_sq(float dx, float dy, float dz) {
 
 }  // namespace
 
-// One warp per group of 32 bodies (kWide: 64, two per lane).
-template <bool kFused, bool kCompensated, bool kRelative, bool kBuckets, bool kWide>
-__global__ void __launch_bounds__(kThreads, walk_min_blocks(kRelative, kWide))
+// One warp per group of 32 bodies (kWide: 64, two per lane).  kFew: the same walk
+// compiled for latency, bit-identical.
+template <bool kFused, bool kCompensated, bool kRelative, bool kBuckets, bool kWide, bool kFew>
+__global__ void __launch_bounds__(kThreads, walk_min_blocks(kRelative, kWide, kFew))
 k_walk(const WalkArgs a) {
     constexpr int kW = kWide ? 64 : 32;
     const float4* __restrict__ pos = a.pos;
@@ -556,7 +572,7 @@ k_walk(const WalkArgs a) {
                     const f32x2 th2 = pack2(thetaSq, thetaSq);
                     // any body fails: the nearest does (rounding is monotonic)
                     float tMin = INFINITY, rMin = INFINITY;
-#pragma unroll 4
+#pragma unroll(kFew ? 16 : 4)  // (16 in every walk: 1% slower with 6 blocks' registers)
                     for (unsigned B = sm + Mem::body; B < sm + Mem::body + 16u * kW; B += 32) {
                         const ulonglong2 xy = lds_2x2(B), zk = lds_2x2(B + 16);
                         const f32x2 dx = sub2(xy.x, nx), dy = sub2(xy.y, ny), dz = sub2(zk.x, nz);
@@ -606,13 +622,23 @@ k_walk(const WalkArgs a) {
                         c = 0;
                     }
                 }
-                int incl = c;
+                int incl = c, pushed;
+                if (kFew && !kBuckets) {
+                    // c <= 8: bit by bit, four ballots at once instead of a chain of
+                    // shuffles (1.5% of a small walk; at 1M bodies 0.3% slower, it
+                    // is more instructions)
+                    const unsigned w0 = __ballot_sync(0xffffffffu, c & 1), w1 = __ballot_sync(0xffffffffu, c & 2);
+                    const unsigned w2 = __ballot_sync(0xffffffffu, c & 4), w3 = __ballot_sync(0xffffffffu, c & 8);
+                    incl += __popc(w0 & lt) + 2 * __popc(w1 & lt) + 4 * __popc(w2 & lt) + 8 * __popc(w3 & lt);
+                    pushed = __popc(w0) + 2 * __popc(w1) + 4 * __popc(w2) + 8 * __popc(w3);
+                } else {
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += y;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += y;
+                    }
+                    pushed = __shfl_sync(0xffffffffu, incl, 31);
                 }
-                const int pushed = __shfl_sync(0xffffffffu, incl, 31);
                 if (top + pushed > stackCap) {
                     overflow = true;
                     break;
@@ -809,7 +835,8 @@ k_kick_drift(float4* __restrict__ pos, float3* __restrict__ vel, const float3* _
 // ---------------------------------------------------------------- launchers
 
 int bh_walk_grid() { return bh_sm_count() * kBlocksPerSm; }
-static_assert(kMinBlocksPlain <= kBlocksPerSm && kMinBlocksRelative <= kBlocksPerSm && kMinBlocksWide <= kBlocksPerSm,
+static_assert(kMinBlocksPlain <= kBlocksPerSm && kMinBlocksRelative <= kBlocksPerSm && kMinBlocksWide <= kBlocksPerSm &&
+                  kMinBlocksFew <= kBlocksPerSm,
               "spill area sizing");
 
 size_t bh_walk_spill_ints() { return (size_t)bh_walk_grid() * kWarpsPerBlock * kSpillPerWarp; }
@@ -837,10 +864,10 @@ static cudaError_t launch_walk_variant(Kernel kernel, const WalkArgs& a, int max
     // sub-partition, half of them plus one are walked at once: the groups come
     // longest first, so a warp that is done takes a short one, and fewer at once
     // leave no half-empty last wave (walk of theta 0.5 disks / Plummer spheres, us
-    // with six warps per sub-partition and with this many: 60,000 bodies 146 / 168
-    // and 143 / 167, 80,000 180 / 199 and 165 / 180, 100,000 206 / 211 and 173 / 195,
-    // 150,000 235 / 250 and 220 / 244; half of them without the one more: 134 / 200
-    // at 60,000, Plummer spheres have a few long groups).
+    // with six warps per sub-partition and with this many, all in 80 registers:
+    // 60,000 bodies 146 / 168 and 143 / 167, 80,000 180 / 199 and 165 / 180, 100,000
+    // 206 / 211 and 173 / 195, 150,000 235 / 250 and 220 / 244; half of them without
+    // the one more: 134 / 200 at 60,000, Plummer spheres have a few long groups).
     const int perGroup = wide ? 64 : 32, sms = bh_sm_count();
     const long long groups = a.groupTable ? a.groups : (a.n + perGroup - 1) / perGroup;
     const long long half = (groups - 1) / (2ll * kWarpsPerBlock * sms) + 1;  // rounded up
@@ -864,18 +891,23 @@ cudaError_t bh_launch_walk(const WalkArgs& in, bool fused, bool compensated, cud
     if (width != 32 && width != 64) return cudaErrorInvalidValue;
     const bool wide = width == 64;
     // one block per resident slot (the spill area is sized for bh_walk_grid(), the largest)
-    const int maxBlocks = walk_min_blocks(a.relative, wide);
-#define BH_WALK_LAUNCH(F, C, R, B, W) \
-    return launch_walk_variant(k_walk<F, C, R, B, W>, a, maxBlocks, W, s)
-#define BH_WALK_BUCKETS(F, C, R)                                   \
-    do {                                                           \
-        if (wide) {                                                \
-            if (buckets) BH_WALK_LAUNCH(F, C, R, true, true);      \
-            else BH_WALK_LAUNCH(F, C, R, false, true);             \
-        } else {                                                   \
-            if (buckets) BH_WALK_LAUNCH(F, C, R, true, false);     \
-            else BH_WALK_LAUNCH(F, C, R, false, false);            \
-        }                                                          \
+    const long long groups = a.groupTable ? a.groups : (a.n + 31) / 32;
+    const bool few = !wide && groups <= (long long)kFewGroupsPerSm * bh_sm_count();
+    const int maxBlocks = walk_min_blocks(a.relative, wide, few);
+#define BH_WALK_LAUNCH(F, C, R, B, W, N) \
+    return launch_walk_variant(k_walk<F, C, R, B, W, N>, a, maxBlocks, W, s)
+#define BH_WALK_BUCKETS(F, C, R)                                      \
+    do {                                                              \
+        if (wide) {                                                   \
+            if (buckets) BH_WALK_LAUNCH(F, C, R, true, true, false);  \
+            else BH_WALK_LAUNCH(F, C, R, false, true, false);         \
+        } else if (few) {                                             \
+            if (buckets) BH_WALK_LAUNCH(F, C, R, true, false, true);  \
+            else BH_WALK_LAUNCH(F, C, R, false, false, true);         \
+        } else {                                                      \
+            if (buckets) BH_WALK_LAUNCH(F, C, R, true, false, false); \
+            else BH_WALK_LAUNCH(F, C, R, false, false, false);        \
+        }                                                             \
     } while (0)
     if (a.relative) {
         if (fused) {
