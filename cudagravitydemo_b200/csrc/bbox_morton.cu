@@ -29,7 +29,7 @@ __device__ __forceinline__ void warp_minmax(float v[6]) {
 
 // Block-wide min/max of v[0..2] and max of v[3..5]; result valid in thread 0.
 __device__ __forceinline__ void block_minmax(float v[6]) {
-    __shared__ float part[kBoxThreads / 32][6];
+    __shared__ float part[32][6];
     warp_minmax(v);
     const int w = threadIdx.x >> 5;
     if (lane_id() == 0)
@@ -48,7 +48,7 @@ __device__ __forceinline__ void block_minmax(float v[6]) {
 // Block-wide sums of v[0..3] in FP64, in a fixed order (deterministic);
 // result valid in thread 0.
 __device__ __forceinline__ void block_sum4(double v[4]) {
-    __shared__ double part[kBoxThreads / 32][4];
+    __shared__ double part[32][4];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -65,6 +65,57 @@ __device__ __forceinline__ void block_sum4(double v[4]) {
             for (int k = 0; k < 4; k++) v[k] += part[j][k];
     }
     __syncthreads();
+}
+
+// The world box of corners v (basicGravity.cu:90-112: extent = max(w, h, d),
+// scale = (2^bits-1)/extent).
+__device__ __forceinline__ DevBox world_box(const float v[6], int bits, int* err) {
+    const float w = __fsub_rn(v[3], v[0]), h = __fsub_rn(v[4], v[1]), d = __fsub_rn(v[5], v[2]);
+    const float extent = fmaxf(w, fmaxf(h, d));
+    const float scale = __fdiv_rn((float)((1u << bits) - 1u), extent);
+    DevBox bx;
+    bx.mn[0] = v[0]; bx.mn[1] = v[1]; bx.mn[2] = v[2];
+    bx.mx[0] = v[3]; bx.mx[1] = v[4]; bx.mx[2] = v[5];
+    bx.extent = extent;
+    bx.scale = scale;
+    bx.extX = w;
+    bx.pad[0] = bx.pad[1] = bx.pad[2] = 0;
+    if (!(extent > 0.0f) || !isfinite(extent) || !(scale > 0.0f) || !isfinite(scale))
+        bh_set_error(err, BH_ERR_DEGENERATE_BOX);
+    return bx;
+}
+
+// The root from its FP64 sums t (m, m x, m y, m z) and corners r.
+__device__ __forceinline__ DevRoot root_of(const double t[4], const float r[6]) {
+    DevRoot rt;
+    rt.mass = t[0];
+    const double inv = t[0] > 0.0 ? 1.0 / t[0] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        rt.com[k] = t[k + 1] * inv;
+        rt.mn[k] = (double)r[k];
+        rt.mx[k] = (double)r[k + 3];
+    }
+    return rt;
+}
+
+// Spreading uses a 256-entry table: spread[b] moves bit k of byte b to bit 3k.
+__device__ __forceinline__ uint32_t spread_byte(uint32_t b) {
+    uint32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) s |= ((b >> k) & 1u) << (3 * k);
+    return s;
+}
+__device__ __forceinline__ uint64_t spread_coord(const uint32_t* spread, uint32_t v) {
+    return (uint64_t)spread[v & 255u] | ((uint64_t)spread[(v >> 8) & 255u] << 24) |
+           ((uint64_t)spread[(v >> 16) & 255u] << 48);
+}
+__device__ __forceinline__ uint64_t morton_key(const uint32_t* spread, const float4 p, float mx, float my, float mz,
+                                               float scale, uint32_t mask) {
+    const uint32_t x = __float2uint_rz(__fmul_rn(__fsub_rn(p.x, mx), scale)) & mask;
+    const uint32_t y = __float2uint_rz(__fmul_rn(__fsub_rn(p.y, my), scale)) & mask;
+    const uint32_t z = __float2uint_rz(__fmul_rn(__fsub_rn(p.z, mz), scale)) & mask;
+    return (spread_coord(spread, x) << 2) | (spread_coord(spread, y) << 1) | spread_coord(spread, z);
 }
 
 }  // namespace
@@ -137,35 +188,12 @@ k_bbox(const float4* __restrict__ pos, int n, float* __restrict__ partials, unsi
 #pragma unroll
             for (int k = 0; k < 4; k++) t[k] += __ldcg(&partials64[b * 4 + k]);
         block_sum4(t);
-        if (threadIdx.x == 0) {
-            DevRoot rt;
-            rt.mass = t[0];
-            const double inv = t[0] > 0.0 ? 1.0 / t[0] : 0.0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                rt.com[k] = t[k + 1] * inv;
-                rt.mn[k] = (double)r[k];
-                rt.mx[k] = (double)r[k + 3];
-            }
-            *root = rt;
-        }
+        if (threadIdx.x == 0) *root = root_of(t, r);
     }
     if (threadIdx.x == 0) {
-        const float w = __fsub_rn(r[3], r[0]), h = __fsub_rn(r[4], r[1]), d = __fsub_rn(r[5], r[2]);
-        const float extent = fmaxf(w, fmaxf(h, d));
-        const float scale = __fdiv_rn((float)((1u << bits) - 1u), extent);
-        DevBox bx;
-        bx.mn[0] = r[0]; bx.mn[1] = r[1]; bx.mn[2] = r[2];
-        bx.mx[0] = r[3]; bx.mx[1] = r[4]; bx.mx[2] = r[5];
-        bx.extent = extent;
-        bx.scale = scale;
-        bx.extX = w;
-        bx.pad[0] = bx.pad[1] = bx.pad[2] = 0;
-        *box = bx;
+        *box = world_box(r, bits, err);
         if (outMin) *outMin = make_float3(r[0], r[1], r[2]);
         if (outMax) *outMax = make_float3(r[3], r[4], r[5]);
-        if (!(extent > 0.0f) || !isfinite(extent) || !(scale > 0.0f) || !isfinite(scale))
-            bh_set_error(err, BH_ERR_DEGENERATE_BOX);
         *ticket = 0u;
     }
     for (int i = threadIdx.x; i < zeroWords; i += blockDim.x) zeroBuf[i] = 0u;
@@ -201,21 +229,7 @@ k_bbox_segments(const float4* __restrict__ pos, const int* __restrict__ segOff, 
         for (; i < hi; i += blockDim.x) take(__ldg(&pos[i]));
         if (bad) bh_set_error(err, BH_ERR_NONFINITE);
         block_minmax(v);
-        if (threadIdx.x == 0) {
-            const float w = __fsub_rn(v[3], v[0]), h = __fsub_rn(v[4], v[1]), d = __fsub_rn(v[5], v[2]);
-            const float extent = fmaxf(w, fmaxf(h, d));
-            const float scale = __fdiv_rn((float)((1u << bits) - 1u), extent);
-            DevBox bx;
-            bx.mn[0] = v[0]; bx.mn[1] = v[1]; bx.mn[2] = v[2];
-            bx.mx[0] = v[3]; bx.mx[1] = v[4]; bx.mx[2] = v[5];
-            bx.extent = extent;
-            bx.scale = scale;
-            bx.extX = w;
-            bx.pad[0] = bx.pad[1] = bx.pad[2] = 0;
-            boxes[sy] = bx;
-            if (!(extent > 0.0f) || !isfinite(extent) || !(scale > 0.0f) || !isfinite(scale))
-                bh_set_error(err, BH_ERR_DEGENERATE_BOX);
-        }
+        if (threadIdx.x == 0) boxes[sy] = world_box(v, bits, err);
     }
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < zeroWords; i += blockDim.x) zeroBuf[i] = 0u;
@@ -224,8 +238,7 @@ k_bbox_segments(const float4* __restrict__ pos, const int* __restrict__ segOff, 
 // Morton keys (tree.cu:343-367 generalised to `bits` bits per axis):
 // grid coordinate = (uint32)((p - min) * scale) masked to `bits` bits; key =
 // interleave with x highest (x<<2 | y<<1 | z per bit); idx[i] = i.
-// Spreading uses a 256-entry table in shared memory: spread[b] moves bit k of
-// byte b to bit 3k.
+// The spreading table is in shared memory.
 //
 // In a batch (sysOf set) body i uses the world box of its system sysOf[i] and
 // the system index goes above the Morton bits: key |= sys << 3*bits, so one
@@ -238,11 +251,6 @@ k_bbox_segments(const float4* __restrict__ pos, const int* __restrict__ segOff, 
 constexpr int kMortonThreads = 256;
 constexpr int kMortonPerThread = 8;
 
-__device__ __forceinline__ uint64_t spread_coord(const uint32_t* spread, uint32_t v) {
-    return (uint64_t)spread[v & 255u] | ((uint64_t)spread[(v >> 8) & 255u] << 24) |
-           ((uint64_t)spread[(v >> 16) & 255u] << 48);
-}
-
 __global__ void __launch_bounds__(kMortonThreads)
 k_morton(const float4* __restrict__ pos, int n, const DevBox* __restrict__ box, worldBox boxVal,
          int bits, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx,
@@ -250,12 +258,7 @@ k_morton(const float4* __restrict__ pos, int n, const DevBox* __restrict__ box, 
     __shared__ uint32_t spread[256];
     __shared__ uint32_t shist[8][256];
     __shared__ __align__(16) uint64_t skeys[kMortonThreads * kMortonPerThread];
-    {
-        uint32_t b = threadIdx.x, s = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) s |= ((b >> k) & 1u) << (3 * k);
-        spread[threadIdx.x] = s;
-    }
+    spread[threadIdx.x] = spread_byte(threadIdx.x);
     if (hist)
         for (int i = threadIdx.x; i < npass * 256; i += blockDim.x) (&shist[0][0])[i] = 0u;
     __syncthreads();
@@ -280,10 +283,7 @@ k_morton(const float4* __restrict__ pos, int n, const DevBox* __restrict__ box, 
                     const DevBox* bx = box + sys;
                     mx = bx->mn[0]; my = bx->mn[1]; mz = bx->mn[2]; sc = bx->scale;
                 }
-                const uint32_t x = __float2uint_rz(__fmul_rn(__fsub_rn(p.x, mx), sc)) & mask;
-                const uint32_t y = __float2uint_rz(__fmul_rn(__fsub_rn(p.y, my), sc)) & mask;
-                const uint32_t z = __float2uint_rz(__fmul_rn(__fsub_rn(p.z, mz), sc)) & mask;
-                key = (spread_coord(spread, x) << 2) | (spread_coord(spread, y) << 1) | spread_coord(spread, z);
+                key = morton_key(spread, p, mx, my, mz, sc, mask);
                 if (sysOf) key |= sys << (3 * bits);
                 keys[i] = key;
                 if (idx) idx[i] = (uint32_t)i;
@@ -325,6 +325,68 @@ k_morton(const float4* __restrict__ pos, int n, const DevBox* __restrict__ box, 
             const uint32_t c = (&shist[0][0])[i];
             if (c) atomicAdd(&hist[i], c);
         }
+    }
+}
+
+// Box and keys of a small system in one block: the bodies stay in registers
+// between the two, and a launch, the partial results and the ticket go.  Bound by
+// latency (a load, two reductions, the keys).  Box and keys by two kernels and
+// by this one, us: 1,000 bodies 15.2 and 10.0, 4,000 17.2 and 10.4 (four bodies a
+// thread), 6,000 17.2 and 13.7, 8,192 17.2 and 14.3 (eight).  Same box and keys; the
+// FP64 sums of the root are in another order.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallMax = 8 * kSmallThreads;
+
+template <int kPerThread>
+__global__ void __launch_bounds__(kSmallThreads)
+k_box_keys_small(const float4* __restrict__ pos, int n, DevBox* box, float3* outMin, float3* outMax, int bits, int* err,
+                 DevRoot* root, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
+    __shared__ uint32_t spread[256];
+    __shared__ DevBox sBox;
+    if (threadIdx.x < 256) spread[threadIdx.x] = spread_byte(threadIdx.x);
+    float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    double m4[4] = {0.0, 0.0, 0.0, 0.0};
+    float4 p[kPerThread];
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < kPerThread; j++) {
+        const int i = j * kSmallThreads + threadIdx.x;
+        if (i < n) p[j] = __ldg(&pos[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < kPerThread; j++) {
+        if (j * kSmallThreads + (int)threadIdx.x >= n) break;
+        bad |= !(isfinite(p[j].x) && isfinite(p[j].y) && isfinite(p[j].z));
+        v[0] = fminf(v[0], p[j].x); v[3] = fmaxf(v[3], p[j].x);
+        v[1] = fminf(v[1], p[j].y); v[4] = fmaxf(v[4], p[j].y);
+        v[2] = fminf(v[2], p[j].z); v[5] = fmaxf(v[5], p[j].z);
+        const double m = p[j].w;
+        m4[0] += m;
+        m4[1] = fma(m, (double)p[j].x, m4[1]);
+        m4[2] = fma(m, (double)p[j].y, m4[2]);
+        m4[3] = fma(m, (double)p[j].z, m4[3]);
+    }
+    if (bad) bh_set_error(err, BH_ERR_NONFINITE);
+    block_minmax(v);
+    if (threadIdx.x == 0) {
+        sBox = world_box(v, bits, err);
+        *box = sBox;
+        if (outMin) *outMin = make_float3(v[0], v[1], v[2]);
+        if (outMax) *outMax = make_float3(v[3], v[4], v[5]);
+    }
+    if (root) {
+        block_sum4(m4);
+        if (threadIdx.x == 0) *root = root_of(m4, v);
+    }
+    __syncthreads();
+    const float mx = sBox.mn[0], my = sBox.mn[1], mz = sBox.mn[2], scale = sBox.scale;
+    const uint32_t mask = (bits >= 32) ? 0xffffffffu : ((1u << bits) - 1u);
+#pragma unroll
+    for (int j = 0; j < kPerThread; j++) {
+        const int i = j * kSmallThreads + threadIdx.x;
+        if (i >= n) break;
+        keys[i] = morton_key(spread, p[j], mx, my, mz, scale, mask);
+        if (idx) idx[i] = (uint32_t)i;
     }
 }
 
@@ -385,6 +447,22 @@ cudaError_t bh_launch_morton(const float4* pos, int n, const DevBox* boxPtr, wor
     grid = grid < 1 ? 1 : grid;
     k_morton<<<grid, kMortonThreads, 0, s>>>(pos, n, boxPtr, boxVal, bits, keys, idx, hist, npass, sysOf);
     return cudaGetLastError();
+}
+
+bool bh_box_keys_one_launch(int n, const uint32_t* hist) { return !hist && n <= kSmallMax; }
+
+cudaError_t bh_launch_box_keys(const float4* pos, int n, float* partials, unsigned* ticket, DevBox* box, float3* outMin,
+                               float3* outMax, int bits, int* err, double* partials64, DevRoot* root, uint64_t* keys,
+                               uint32_t* idx, uint32_t* hist, int npass, cudaStream_t s) {
+    if (bh_box_keys_one_launch(n, hist)) {
+        const auto kernel = n <= 4 * kSmallThreads ? k_box_keys_small<4> : k_box_keys_small<8>;
+        kernel<<<1, kSmallThreads, 0, s>>>(pos, n, box, outMin, outMax, bits, err, root, keys, idx);
+        return cudaGetLastError();
+    }
+    const cudaError_t e = bh_launch_bbox(pos, n, partials, ticket, box, outMin, outMax, bits, err, hist,
+                                         hist ? npass * 256 : 0, s, partials64, root);
+    const worldBox none = {0, 0, 0, 0, 0};
+    return e != cudaSuccess ? e : bh_launch_morton(pos, n, box, none, bits, keys, idx, hist, npass, s);
 }
 
 cudaError_t bh_launch_bbox_segments(const float4* pos, const int* segOff, int systems, DevBox* boxes, int bits,

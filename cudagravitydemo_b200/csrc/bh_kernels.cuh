@@ -17,6 +17,12 @@ cudaError_t bh_launch_bbox(const float4* pos, int n, float* partials, unsigned* 
 cudaError_t bh_launch_morton(const float4* pos, int n, const DevBox* boxPtr, worldBox boxVal, int bits,
                              uint64_t* keys, uint32_t* idx, uint32_t* hist, int npass, cudaStream_t s,
                              const uint16_t* sysOf = nullptr);
+// Box and keys of one system (as the two above, which it launches unless one
+// block can do both: few bodies, and nobody needs the histograms).
+bool bh_box_keys_one_launch(int n, const uint32_t* hist);
+cudaError_t bh_launch_box_keys(const float4* pos, int n, float* partials, unsigned* ticket, DevBox* box, float3* outMin,
+                               float3* outMax, int bits, int* err, double* partials64, DevRoot* root, uint64_t* keys,
+                               uint32_t* idx, uint32_t* hist, int npass, cudaStream_t s);
 // Batch: per-system world boxes (systems blocks at most) and zeroed histograms.
 cudaError_t bh_launch_bbox_segments(const float4* pos, const int* segOff, int systems, DevBox* boxes, int bits,
                                     int* err, uint32_t* zeroBuf, int zeroWords, cudaStream_t s);

@@ -405,12 +405,9 @@ extern "C" int bh_build_tree(treeState* st, float4** pos, float3** vel, cudaStre
 #define TRYC(x) TRY(((x) == cudaSuccess) ? BH_OK : bh_note_cuda_error(cudaGetLastError()))
     TRY(cudaMemsetAsync(c->err, 0, sizeof(int), s) == cudaSuccess ? BH_OK : BH_ERR_CUDA);
     uint32_t* const hist = ctx_sort_histogram(c, n);
-    // stage 1: world box (basicGravity.cu:143-155)
-    TRYC(bh_launch_bbox(*pos, n, c->bboxPartials, c->bboxTicket, c->box, st->boundingData[2], st->boundingData[3],
-                        bits, c->err, hist, hist ? 8 * 256 : 0, s, c->bboxPartials64, c->root64));
-    // stage 2: keys (basicGravity.cu:176-183)
-    worldBox none = {0, 0, 0, 0, 0};
-    TRYC(bh_launch_morton(*pos, n, c->box, none, bits, st->mortonIn, st->indexIn, hist, 8, s));
+    // stages 1 and 2: world box (basicGravity.cu:143-155) and keys (basicGravity.cu:176-183)
+    TRYC(bh_launch_box_keys(*pos, n, c->bboxPartials, c->bboxTicket, c->box, st->boundingData[2], st->boundingData[3],
+                            bits, c->err, c->bboxPartials64, c->root64, st->mortonIn, st->indexIn, hist, 8, s));
     // stage 3: sort + reorder + pointer swap (basicGravity.cu:190-226)
     TRY(ctx_sort(c, st->mortonIn, st->indexIn, st->mortonOut, st->indexOut, n, 64, true, s));
     TRYC(bh_launch_reorder(*pos, *vel, nullptr, st->indexOut, st->sortedPosMassVals, st->sortedVelVals, nullptr,
@@ -1087,16 +1084,15 @@ static int sim_enqueue_build(bh_sim* s, cudaEvent_t* ev, cudaEvent_t afterReorde
     const int npass = (keyBits + 7) / 8;
     cudaStream_t st = s->stream;
     uint32_t* const hist = ctx_sort_histogram(c, n);
-    const int histWords = hist ? npass * 256 : 0;
     if (ev) BH_CUDA_TRY(cudaEventRecord(ev[0], st));
-    worldBox none = {0, 0, 0, 0, 0};
     if (s->systems) {
-        BH_CUDA_TRY(bh_launch_bbox_segments(s->posA, s->segOff, s->systems, s->boxes, bits, c->err, hist, histWords, st));
+        const worldBox none = {0, 0, 0, 0, 0};
+        BH_CUDA_TRY(bh_launch_bbox_segments(s->posA, s->segOff, s->systems, s->boxes, bits, c->err, hist,
+                                            hist ? npass * 256 : 0, st));
         BH_CUDA_TRY(bh_launch_morton(s->posA, n, s->boxes, none, bits, s->keysA, nullptr, hist, npass, st, s->sysOf));
     } else {
-        BH_CUDA_TRY(bh_launch_bbox(s->posA, n, c->bboxPartials, c->bboxTicket, c->box, s->corner, s->corner + 1,
-                                   bits, c->err, hist, histWords, st, c->bboxPartials64, c->root64));
-        BH_CUDA_TRY(bh_launch_morton(s->posA, n, c->box, none, bits, s->keysA, nullptr, hist, npass, st));
+        BH_CUDA_TRY(bh_launch_box_keys(s->posA, n, c->bboxPartials, c->bboxTicket, c->box, s->corner, s->corner + 1,
+                                       bits, c->err, c->bboxPartials64, c->root64, s->keysA, nullptr, hist, npass, st));
     }
     if (ev) BH_CUDA_TRY(cudaEventRecord(ev[1], st));
     int rc = ctx_sort(c, s->keysA, nullptr, s->keysB, s->perm, n, keyBits, true, st);
@@ -1238,9 +1234,11 @@ static int sim_enqueue_step(bh_sim* s, cudaEvent_t* ev) {
 extern "C" int bh_sim_kernels_per_step(const bh_sim* s) {
     if (!s) return 0;
     const int digits = (3 * sim_bits(s) + (s->systems ? s->sysBits : 0) + 7) / 8;
-    const int npass = (s->n > 0 ? s->n : s->capacity) <= bh_sort_cluster_limit() ? 1 : digits;
-    return 2 /* box, keys */ + npass /* sort */ + 1 /* reorder */ + 4 /* tree */ + (s->prm.exportNodes ? 1 : 0) +
-           (s->prm.macMode == 2 ? 2 : 0) /* features, selection */ + 2 /* group order */ + 1 /* walk */;
+    const int n = s->n > 0 ? s->n : s->capacity;
+    const int npass = n <= bh_sort_cluster_limit() ? 1 : digits;
+    const bool together = !s->systems && bh_box_keys_one_launch(n, ctx_sort_histogram(s->ctx, n));
+    return (together ? 1 : 2) /* box, keys */ + npass /* sort */ + 1 /* reorder */ + 4 /* tree */ +
+           (s->prm.exportNodes ? 1 : 0) + (s->prm.macMode == 2 ? 2 : 0) /* features, selection */ + 2 /* group order */ + 1 /* walk */;
 }
 
 // nsteps real steps issued stage by stage (no graph, each queued behind a
