@@ -8,6 +8,8 @@
 // Every sum is in double precision; W is the exact O(N^2) pair sum.  Block
 // partials are reduced by one block in a fixed order, so results are
 // deterministic for a given launch geometry.
+#include <type_traits>
+
 #include "bh_internal.cuh"
 #include "rsqrt64.cuh"
 
@@ -86,38 +88,43 @@ k_diag_potential(const float4* __restrict__ pos, int n, int rows, int perPart, d
         id[k] = row * kRow + k * kPotThreads + threadIdx.x;
         const float4 p = id[k] < n ? pos[id[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
         x[k] = p.x; y[k] = p.y; z[k] = p.z; m[k] = p.w;
-        phi[k] = 0.0;
     }
     const int most = rows / 2;  // tiles at distance 0 .. most
     const int lo = blockIdx.y * perPart, hi = lo + perPart < most + 1 ? lo + perPart : most + 1;
-    for (int d = lo; d < hi; d++) {
-        if (d > 0 && 2 * d == rows && row >= d) break;  // the opposite row has this pair
-        const int other = row + d < rows ? row + d : row + d - rows;
-        const int base = other * kRow, cnt = n - base < kRow ? n - base : kRow;
-        __syncthreads();
-        for (int j = threadIdx.x; j < cnt; j += kPotThreads) {
-            const float4 p = pos[base + j];
-            tile[j][0] = make_double2(p.x, p.y);
-            tile[j][1] = make_double2(p.z, p.w);
-        }
-        __syncthreads();
-        auto add = [&](int j, bool own) {
-            const double2 xy = tile[j][0], zm = tile[j][1];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const double dx = xy.x - x[k], dy = xy.y - y[k], dz = zm.x - z[k];
-                const double t = mass_over_r(zm.y, fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
-                phi[k] += own && base + j <= id[k] ? 0.0 : t;
+    auto sum = [&](auto edges) {
+        phi[0] = phi[1] = 0.0;
+        for (int d = lo; d < hi; d++) {
+            if (d > 0 && 2 * d == rows && row >= d) break;  // the opposite row has this pair
+            const int other = row + d < rows ? row + d : row + d - rows;
+            const int base = other * kRow, cnt = n - base < kRow ? n - base : kRow;
+            __syncthreads();
+            for (int j = threadIdx.x; j < cnt; j += kPotThreads) {
+                const float4 p = pos[base + j];
+                tile[j][0] = make_double2(p.x, p.y);
+                tile[j][1] = make_double2(p.z, p.w);
             }
-        };
-        if (d == 0) {
-            for (int j = 0; j < cnt; j++) add(j, true);
-        } else {
+            __syncthreads();
+            auto add = [&](int j, bool own) {
+                const double2 xy = tile[j][0], zm = tile[j][1];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const double dx = xy.x - x[k], dy = xy.y - y[k], dz = zm.x - z[k];
+                    const double t = mass_over_r<decltype(edges)::value>(zm.y, fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+                    phi[k] += own && base + j <= id[k] ? 0.0 : t;
+                }
+            };
+            if (d == 0) {
+                for (int j = 0; j < cnt; j++) add(j, true);
+            } else {
 #pragma unroll 4
-            for (int j = 0; j < cnt; j++) add(j, false);
+                for (int j = 0; j < cnt; j++) add(j, false);
+            }
         }
-    }
-    double v[1] = {(id[0] < n ? m[0] * phi[0] : 0.0) + (id[1] < n ? m[1] * phi[1] : 0.0)};
+        return (id[0] < n ? m[0] * phi[0] : 0.0) + (id[1] < n ? m[1] * phi[1] : 0.0);
+    };
+    double v[1] = {sum(std::false_type())};
+    // a pair at distance 0 or infinity: once more, with these
+    if (__syncthreads_or(!isfinite(v[0]))) v[0] = sum(std::true_type());
     block_sum<1, kPotThreads>(v);
     if (threadIdx.x == 0) partial[(size_t)blockIdx.y * rows + row] = v[0];
 }

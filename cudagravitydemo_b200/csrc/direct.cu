@@ -114,6 +114,8 @@ extern "C" int bh_direct_sum_f64(const float4* pos, int n, const int* targets, i
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_direct_f64, pos, n, targets, ntargets, eps * eps, G, acc);
+    // (from 1e300 on every acceleration is 0 in double precision; the series wants it finite)
+    const double eps2 = eps * eps < 1e300 || eps != eps ? eps * eps : 1e300;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_direct_f64, pos, n, targets, ntargets, eps2, G, acc);
     return e == cudaSuccess ? BH_OK : bh_note_cuda_error(e);
 }

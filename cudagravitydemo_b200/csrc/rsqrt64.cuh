@@ -14,7 +14,7 @@ __device__ __forceinline__ double rsqrt64_seed(double x) {
     return y;
 }
 
-// m / x^(3/2)
+// m / x^(3/2), 0 < x < inf
 __device__ __forceinline__ double mass_over_r3(double m, double x) {
     const double y = rsqrt64_seed(x), y2 = y * y;
     const double h = fma(-x, y2, 1.0);
@@ -22,10 +22,14 @@ __device__ __forceinline__ double mass_over_r3(double m, double x) {
     return fma(f, h * fma(1.875, h, 1.5), f);
 }
 
-// m / sqrt(x)
+// m / sqrt(x), 0 < x < inf; with kEdges also x = 0 and x = inf, where h is not a
+// number: a small one in its place lets y = inf and y = 0 come through the series
+// (5% of a pair sum, so the sums ask for it only when they have to).
+template <bool kEdges>
 __device__ __forceinline__ double mass_over_r(double m, double x) {
     const double y = rsqrt64_seed(x);
-    const double h = fma(-x, y * y, 1.0);
+    double h = fma(-x, y * y, 1.0);
+    if (kEdges) h = __hiloint2double(__double2hiint(h) & 0x40000000 ? 0x3e000000 : __double2hiint(h), __double2loint(h));
     const double f = m * y;
     return fma(f, h * fma(0.375, h, 0.5), f);
 }

@@ -54,3 +54,21 @@ def test_pair_potential_edges(torch_cuda, engine, n):
         w[np.arange(w.shape[0]), np.arange(i, i + w.shape[0])] = 0.0
         want -= w.sum()
     assert got == pytest.approx(want, rel=TOL, abs=0)
+
+
+@pytest.mark.parametrize("n", [40, 300, 1000])
+def test_infinite_and_zero_distances(torch_cuda, engine, n):
+    from cudagravitydemo_b200 import accuracy
+    torch = torch_cuda
+    v = torch.zeros((n, 3), device="cuda")
+    p = _bodies(n, n + 2)
+    p[3, :3] = p[n - 1, :3]  # without softening a coincident pair is bound without limit
+    assert engine.diagnostics(torch.from_numpy(p).cuda(), v, 0.0, 1.0)["potential"] == -np.inf
+    far = _bodies(n, n + 2)
+    far[n - 2, 0] = np.inf  # a body infinitely far away adds nothing
+    gone = np.delete(far, n - 2, axis=0)
+    got = engine.diagnostics(torch.from_numpy(far).cuda(), v, 0.01, 1.0)["potential"]
+    want = engine.diagnostics(torch.from_numpy(gone).cuda(), v[1:], 0.01, 1.0)["potential"]
+    assert got == pytest.approx(want, rel=TOL, abs=0)
+    t = torch.arange(n, dtype=torch.int32, device="cuda")
+    assert not accuracy.direct_sum(torch.from_numpy(p).cuda(), t, np.inf, 1.0).any()  # softened away
