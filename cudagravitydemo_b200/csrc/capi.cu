@@ -292,14 +292,22 @@ static int ctx_sort(bh_ctx* c, const uint64_t* keysIn, const uint32_t* valsIn, u
 static int ctx_build(bh_ctx* c, const uint64_t* sortedKeys, const float4* sortedPos, int n, int bits,
                      node* exportTo, cudaStream_t s, cudaEvent_t* ev = nullptr, const DevBox* boxes = nullptr,
                      cudaEvent_t beforeMass = nullptr) {
-    const int blocks = (n + bh_tree_threads() - 1) / bh_tree_threads();
-    BH_CUDA_TRY(bh_launch_tree_count(sortedKeys, n, bits, c->delta, c->blockLevel, s));
-    if (ev) BH_CUDA_TRY(cudaEventRecord(ev[0], s));
-    BH_CUDA_TRY(bh_launch_tree_scan(c->blockLevel, blocks, n, bits, c->maxNodes, c->box, c->info, c->nCB,
-                                    c->levelTotal, c->scanTicket, c->err, s));
-    if (ev) BH_CUDA_TRY(cudaEventRecord(ev[1], s));
-    BH_CUDA_TRY(bh_launch_tree_nodes(sortedKeys, c->delta, n, bits, c->blockLevel, c->info, c->maxNodes,
-                                     boxes ? boxes : c->box, c->nCB, c->nParent, c->nFirst, c->nMeta, s));
+    const DevBox* const extents = boxes ? boxes : c->box;
+    if (bh_tree_build_one_launch(n)) {  // (all of it before the first event)
+        BH_CUDA_TRY(bh_launch_tree_build_small(sortedKeys, n, bits, c->maxNodes, c->box, extents, c->delta, c->info,
+                                               c->nCB, c->nParent, c->nFirst, c->nMeta, c->err, s));
+        if (ev) BH_CUDA_TRY(cudaEventRecord(ev[0], s));
+        if (ev) BH_CUDA_TRY(cudaEventRecord(ev[1], s));
+    } else {
+        const int blocks = (n + bh_tree_threads() - 1) / bh_tree_threads();
+        BH_CUDA_TRY(bh_launch_tree_count(sortedKeys, n, bits, c->delta, c->blockLevel, s));
+        if (ev) BH_CUDA_TRY(cudaEventRecord(ev[0], s));
+        BH_CUDA_TRY(bh_launch_tree_scan(c->blockLevel, blocks, n, bits, c->maxNodes, c->box, c->info, c->nCB,
+                                        c->levelTotal, c->scanTicket, c->err, s));
+        if (ev) BH_CUDA_TRY(cudaEventRecord(ev[1], s));
+        BH_CUDA_TRY(bh_launch_tree_nodes(sortedKeys, c->delta, n, bits, c->blockLevel, c->info, c->maxNodes, extents,
+                                         c->nCB, c->nParent, c->nFirst, c->nMeta, s));
+    }
     if (ev) BH_CUDA_TRY(cudaEventRecord(ev[2], s));
     if (beforeMass) BH_CUDA_TRY(cudaStreamWaitEvent(s, beforeMass, 0));
     BH_CUDA_TRY(bh_launch_tree_mass(sortedPos, c->delta, n, bits, c->info, c->nCB, c->nCom, c->wn, c->nFirst,
@@ -1237,7 +1245,7 @@ extern "C" int bh_sim_kernels_per_step(const bh_sim* s) {
     const int n = s->n > 0 ? s->n : s->capacity;
     const int npass = n <= bh_sort_cluster_limit() ? 1 : digits;
     const bool together = !s->systems && bh_box_keys_one_launch(n, ctx_sort_histogram(s->ctx, n));
-    return (together ? 1 : 2) /* box, keys */ + npass /* sort */ + 1 /* reorder */ + 4 /* tree */ +
+    return (together ? 1 : 2) /* box, keys */ + npass /* sort */ + 1 /* reorder */ + (bh_tree_build_one_launch(n) ? 2 : 4) /* tree */ +
            (s->prm.exportNodes ? 1 : 0) + (s->prm.macMode == 2 ? 2 : 0) /* features, selection */ + 2 /* group order */ + 1 /* walk */;
 }
 

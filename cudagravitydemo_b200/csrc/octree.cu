@@ -53,6 +53,22 @@ __device__ __forceinline__ int common_levels(uint64_t a, uint64_t b, int bits) {
     return bits - 1 - h / 3;
 }
 
+// The levels where a body with a and b common levels with its neighbours
+// starts nodes: [lo, hi] below the root (empty when lo > hi), and level 0 when
+// root.
+struct NodeLevels {
+    int lo = 1, hi = 0;
+    bool root = false;
+};
+__device__ __forceinline__ NodeLevels node_levels(int a, int b, int bits) {
+    NodeLevels v;
+    v.root = a < 0;
+    v.lo = a + 1 < 1 ? 1 : a + 1;
+    v.hi = (a > b ? a : b) + 1;
+    v.hi = v.hi > bits ? bits : v.hi;
+    return v;
+}
+
 // delta[] stores common_levels with the left neighbour, 0xff for -1.
 __device__ __forceinline__ int delta_levels(const uint8_t* delta, int i) {
     const int d = delta[i];
@@ -79,10 +95,10 @@ k_tree_count(const uint64_t* __restrict__ keys, int n, int bits, uint8_t* __rest
         const int a = (i > 0) ? common_levels(keys[i - 1], k, bits) : -1;
         const int b = (i + 1 < n) ? common_levels(k, keys[i + 1], bits) : -1;
         delta[i] = (uint8_t)(a < 0 ? 0xff : a);
-        root = a < 0;
-        lo = a + 1 < 1 ? 1 : a + 1;
-        hi = (a > b ? a : b) + 1;
-        hi = hi > bits ? bits : hi;
+        const NodeLevels v = node_levels(a, b, bits);
+        root = v.root;
+        lo = v.lo;
+        hi = v.hi;
     }
     {
         const unsigned m = __ballot_sync(0xffffffffu, root);
@@ -97,6 +113,40 @@ k_tree_count(const uint64_t* __restrict__ keys, int n, int bits, uint8_t* __rest
     }
     __syncthreads();
     if (tid < BH_LEVEL_SLOTS) blockLevel[tid * gridDim.x + blockIdx.x] = cnt[tid];
+}
+
+// The level table from c, the nodes of level `lane`, by one warp: offset (nodes
+// before this level) in every lane, true when the tree fits.  One level per lane
+// (in one thread, level after level, it took a third of the kernel's own time:
+// 10.4 -> 8.6 us between events at 1,000 bodies)
+__device__ __forceinline__ bool level_table(int c, int bits, int maxNodes, const DevBox* __restrict__ box,
+                                            DevTreeInfo* info, int2* nCB, int* err, int& offset) {
+    const int lane = lane_id();
+    int after = c;  // nodes up to and including this level
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, after, o);
+        if (lane >= o) after += y;
+    }
+    const int nodes = __shfl_sync(0xffffffffu, after, 31);
+    const unsigned used = __ballot_sync(0xffffffffu, c > 0), over = __ballot_sync(0xffffffffu, c > 0 && after > maxNodes);
+    const int overflow = over ? __ffs(over) - 1 : 0;
+    offset = after - c;
+    if (lane < BH_LEVEL_SLOTS) {
+        info->levelOffset[lane] = offset;
+        info->levelCount[lane] = c;
+        const float sz = ldexpf(box->extX, -lane);  // exact: extX / 2^level; the first system's (the only one outside a batch)
+        info->sizeSq[lane] = __fmul_rn(sz, sz);
+    }
+    if (lane == 0) {
+        info->deepest = used ? 31 - __clz(used) : 0;
+        info->nodeCount = nodes;
+        info->overflowLevel = overflow;
+        info->pad = 0;
+        if (overflow) bh_set_error(err, BH_ERR_TREE_OVERFLOW);
+        else nCB[nodes].x = nodes;  // sentinel: end of the last child range
+    }
+    return overflow == 0;
 }
 
 // Pass 2 (one block per level): blockLevel[L][b] (level-major) -> exclusive
@@ -161,33 +211,64 @@ k_tree_scan(int* __restrict__ blockLevel, int nblocks, int n, int bits, int maxN
     }
     __syncthreads();
     if (!last || w != 0) return;
-    // one level per lane (in one thread, level after level, it took a third of
-    // the kernel's own time: 10.4 -> 8.6 us between events at 1,000 bodies)
     __threadfence();
     const int c = lane <= bits ? __ldcg(&levelTotal[lane]) : 0;
-    int after = c;  // nodes up to and including this level
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, after, o);
-        if (lane >= o) after += y;
-    }
-    const int nodes = __shfl_sync(0xffffffffu, after, 31);
-    const unsigned used = __ballot_sync(0xffffffffu, c > 0), over = __ballot_sync(0xffffffffu, c > 0 && after > maxNodes);
-    const int overflow = over ? __ffs(over) - 1 : 0;
-    if (lane < BH_LEVEL_SLOTS) {
-        info->levelOffset[lane] = after - c;
-        info->levelCount[lane] = c;
-        const float sz = ldexpf(box->extX, -lane);  // exact: extX / 2^level; the first system's (the only one outside a batch)
-        info->sizeSq[lane] = __fmul_rn(sz, sz);
-    }
-    if (lane == 0) {
-        info->deepest = used ? 31 - __clz(used) : 0;
-        info->nodeCount = nodes;
-        info->overflowLevel = overflow;
-        info->pad = 0;
-        if (overflow) bh_set_error(err, BH_ERR_TREE_OVERFLOW);
-        else nCB[nodes].x = nodes;  // sentinel: end of the last child range
-        *ticket = 0u;               // re-armed for the next build
+    int offset;
+    level_table(c, bits, maxNodes, box, info, nCB, err, offset);
+    if (lane == 0) *ticket = 0u;  // re-armed for the next build
+}
+
+// Does a body with levels v start a node at level L?
+__device__ __forceinline__ bool starts(const NodeLevels& v, int L) {
+    return L == 0 ? v.root : (L >= v.lo && L <= v.hi);
+}
+// The levels where some body of the warp starts a node: [wlo, whi] (empty when
+// wlo > whi); every other level has no flag in this warp.
+__device__ __forceinline__ void warp_levels(const NodeLevels& v, int bits, int& wlo, int& whi) {
+    wlo = __reduce_min_sync(0xffffffffu, v.lo <= v.hi ? v.lo : bits + 1);
+    whi = __reduce_max_sync(0xffffffffu, v.lo <= v.hi ? v.hi : 0);
+    if (__any_sync(0xffffffffu, v.root)) wlo = 0;
+}
+// x-extent of the system that a key belongs to
+__device__ __forceinline__ float system_extent(const DevBox* __restrict__ boxes, uint64_t key, int bits) {
+    const int shift = 3 * bits;
+    return boxes[shift >= 64 ? 0 : (int)(key >> shift)].extX;
+}
+
+// The nodes that the bodies of a warp start.  off: per level, how many nodes of
+// it the warps before this one start.
+__device__ __forceinline__ void write_nodes(int i, uint64_t key, float extX, const NodeLevels& lv, int wlo,
+                                            int whi, const int* off, const int* levelOff, int bits, int maxNodes,
+                                            int nodeCount, int2* __restrict__ nCB, int* __restrict__ nParent,
+                                            int* __restrict__ nFirst, int* __restrict__ nMeta) {
+    // walk the levels keeping r_{L-2}, r_{L-1}, r_L; node L-1 is complete at
+    // L.  Below wlo no body of the warp has a flag, so its ranks there are the
+    // warp's offset alone; the walk starts at wlo and ends at whi + 1 (the
+    // child ranges of the level-whi nodes).
+    if (wlo > whi) return;  // uniform: this warp starts no node
+    int r2 = 0, r1 = 0, f2 = 0, f1 = 0;
+    if (wlo >= 2) r2 = off[wlo - 2];
+    if (wlo >= 1) r1 = off[wlo - 1];
+    const unsigned lt = lanemask_lt();
+    for (int L = wlo; L <= whi + 1; L++) {
+        const bool f = starts(lv, L);
+        const unsigned m = (L <= whi) ? __ballot_sync(0xffffffffu, f) : 0u;
+        const int r = off[L] + __popc(m & lt);
+        const int Ln = L - 1;  // node level completed in this iteration
+        if (Ln >= 0 && f1) {
+            const int idx = levelOff[Ln] + r1;
+            const int parent = (Ln == 0) ? -1 : levelOff[Ln - 1] + r2 + f2 - 1;
+            const int childBegin = levelOff[L] + r;
+            if (idx < maxNodes && idx < nodeCount) {
+                const float sz = ldexpf(extX, -Ln);  // exact: extX / 2^L
+                nCB[idx] = make_int2(childBegin, __float_as_int(__fmul_rn(sz, sz)));
+                nParent[idx] = parent;
+                nFirst[idx] = i;
+                nMeta[idx] = Ln | ((int)(level_prefix(key, bits, Ln) & 7ull) << 8);
+            }
+        }
+        r2 = r1; f2 = f1;
+        r1 = r; f1 = f;
     }
 }
 
@@ -218,39 +299,28 @@ k_tree_nodes(const uint64_t* __restrict__ keys, const uint8_t* __restrict__ delt
     }
     const int i = blockIdx.x * kTreeThreads + tid;
     const bool valid = i < n;
-    int lo = 1, hi = 0;  // node levels of body i (empty range when lo > hi)
-    bool root = false;   // body i starts a root
+    NodeLevels lv;
     uint64_t key = 0;
     float extX = 0.f;
     if (valid) {
         key = keys[i];
         const int a = (i > 0) ? delta_levels(delta, i) : -1;
         const int b = (i + 1 < n) ? delta_levels(delta, i + 1) : -1;
-        root = a < 0;
-        lo = a + 1 < 1 ? 1 : a + 1;
-        hi = (a > b ? a : b) + 1;
-        hi = hi > bits ? bits : hi;
-        const int shift = 3 * bits;
-        extX = boxes[shift >= 64 ? 0 : (int)(key >> shift)].extX;
+        lv = node_levels(a, b, bits);
+        extX = system_extent(boxes, key, bits);
     }
-    // flag of level L for this body (level 0: a root)
-    auto flag = [&](int L) -> bool { return valid && (L == 0 ? root : (L >= lo && L <= hi)); };
-    // the levels where some body of the warp starts a node: [wlo, whi]
-    // (empty when wlo > whi); every other level has no flag in this warp
-    const bool anyRoot = __any_sync(0xffffffffu, valid && root);
-    int wlo = __reduce_min_sync(0xffffffffu, valid && lo <= hi ? lo : bits + 1);
-    const int whi = __reduce_max_sync(0xffffffffu, valid && lo <= hi ? hi : 0);
-    if (anyRoot) wlo = 0;
+    int wlo, whi;
+    warp_levels(lv, bits, wlo, whi);
     // warp totals per level
     if (lane <= bits + 1) warpCnt[w][lane] = 0;
     __syncwarp();
     for (int L = wlo; L <= whi; L++) {
-        const unsigned m = __ballot_sync(0xffffffffu, flag(L));
+        const unsigned m = __ballot_sync(0xffffffffu, starts(lv, L));
         if (lane == 0) warpCnt[w][L] = __popc(m);
     }
     __syncthreads();
-    if (tid <= bits + 1) {  // exclusive scan over warps, per level
-        int s = 0;
+    if (tid <= bits + 1) {  // exclusive scan over warps, per level, from the block's offset
+        int s = blockOff[tid];
         for (int k = 0; k < kTreeWarps; k++) {
             const int c = warpCnt[k][tid];
             warpCnt[k][tid] = s;
@@ -258,35 +328,8 @@ k_tree_nodes(const uint64_t* __restrict__ keys, const uint8_t* __restrict__ delt
         }
     }
     __syncthreads();
-    // walk the levels keeping r_{L-2}, r_{L-1}, r_L; node L-1 is complete at
-    // L.  Below wlo no body of the warp has a flag, so its ranks there are the
-    // warp's offsets alone; the walk starts at wlo and ends at whi + 1 (the
-    // child ranges of the level-whi nodes).
-    if (wlo > whi) return;  // uniform: this warp starts no node
-    int r2 = 0, r1 = 0, f2 = 0, f1 = 0;
-    if (wlo >= 2) r2 = blockOff[wlo - 2] + warpCnt[w][wlo - 2];
-    if (wlo >= 1) r1 = blockOff[wlo - 1] + warpCnt[w][wlo - 1];
-    const unsigned lt = lanemask_lt();
-    for (int L = wlo; L <= whi + 1; L++) {
-        const bool f = flag(L);
-        const unsigned m = (L <= whi) ? __ballot_sync(0xffffffffu, f) : 0u;
-        const int r = blockOff[L] + warpCnt[w][L] + __popc(m & lt);
-        const int Ln = L - 1;  // node level completed in this iteration
-        if (Ln >= 0 && f1) {
-            const int idx = levelOff[Ln] + r1;
-            const int parent = (Ln == 0) ? -1 : levelOff[Ln - 1] + r2 + f2 - 1;
-            const int childBegin = levelOff[L] + r;
-            if (idx < maxNodes && idx < nodeCount) {
-                const float sz = ldexpf(extX, -Ln);  // exact: extX / 2^L
-                nCB[idx] = make_int2(childBegin, __float_as_int(__fmul_rn(sz, sz)));
-                nParent[idx] = parent;
-                nFirst[idx] = i;
-                nMeta[idx] = Ln | ((int)(level_prefix(key, bits, Ln) & 7ull) << 8);
-            }
-        }
-        r2 = r1; f2 = f1;
-        r1 = r; f1 = f;
-    }
+    write_nodes(i, key, extX, lv, wlo, whi, warpCnt[w], levelOff, bits, maxNodes, nodeCount, nCB, nParent, nFirst,
+                nMeta);
 }
 
 // Pass 4: upward pass, level by level from the deepest, in one cooperative
@@ -431,6 +474,89 @@ k_tree_mass(const float4* __restrict__ pos, const uint8_t* __restrict__ delta, i
                 grid_barrier(bar, target, err);
             }
         }
+    }
+}
+
+// Count, level table and nodes of a small tree in one block: two launches, the
+// block counts and the ticket go.  Bound by latency.  The three stages between
+// events and this one, us: 1,000 bodies 25.5 and 17.2, 2,000 25.9 and 21.1; with four
+// bodies a thread 4,000 take 24.6 and 27.7.
+constexpr int kBuildThreads = 1024;
+constexpr int kBuildTiles = 2;
+constexpr int kBuildBodies = kBuildThreads * kBuildTiles;
+
+__global__ void __launch_bounds__(kBuildThreads)
+k_tree_build_small(const uint64_t* __restrict__ keys, int n, int bits, int maxNodes, const DevBox* __restrict__ box,
+                   const DevBox* __restrict__ boxes, uint8_t* __restrict__ delta, DevTreeInfo* info,
+                   int2* __restrict__ nCB, int* __restrict__ nParent, int* __restrict__ nFirst, int* __restrict__ nMeta,
+                   int* err) {
+    // nodes per warp and level, then their sums before the warp (odd rows: columns without bank conflicts)
+    __shared__ int off[kBuildTiles * 32][BH_LEVEL_SLOTS + 1];
+    __shared__ int levelTotal[BH_LEVEL_SLOTS], levelOff[BH_LEVEL_SLOTS];
+    __shared__ int sNodes;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int tiles = (n + kBuildThreads - 1) / kBuildThreads;
+    NodeLevels lv[kBuildTiles];
+    uint64_t key[kBuildTiles];
+#pragma unroll
+    for (int t = 0; t < kBuildTiles; t++) {
+        if (t >= tiles) break;
+        const int i = t * kBuildThreads + tid;
+        key[t] = 0;
+        if (i < n) {
+            key[t] = keys[i];
+            const int a = (i > 0) ? common_levels(keys[i - 1], key[t], bits) : -1;
+            const int b = (i + 1 < n) ? common_levels(key[t], keys[i + 1], bits) : -1;
+            delta[i] = (uint8_t)(a < 0 ? 0xff : a);
+            lv[t] = node_levels(a, b, bits);
+        }
+        int* const mine = off[t * 32 + w];
+        if (lane < BH_LEVEL_SLOTS) mine[lane] = 0;
+        __syncwarp();
+        int wlo, whi;
+        warp_levels(lv[t], bits, wlo, whi);
+        for (int L = wlo; L <= whi; L++) {
+            const unsigned m = __ballot_sync(0xffffffffu, starts(lv[t], L));
+            if (lane == 0) mine[L] = __popc(m);
+        }
+    }
+    __syncthreads();
+    if (w < BH_LEVEL_SLOTS) {  // warp w: exclusive scan of level w over the warps
+        int carry = 0;
+        for (int t = 0; t < tiles; t++) {
+            const int c = off[t * 32 + lane][w];
+            int x = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            off[t * 32 + lane][w] = carry + x - c;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) levelTotal[w] = carry;
+    }
+    __syncthreads();
+    if (w == 0) {
+        int offset;
+        const int c = lane <= bits ? levelTotal[lane] : 0;
+        const bool fits = level_table(c, bits, maxNodes, box, info, nCB, err, offset);
+        if (lane < BH_LEVEL_SLOTS) levelOff[lane] = offset;
+        const int nodes = __shfl_sync(0xffffffffu, offset + c, 31);
+        if (lane == 0) sNodes = fits ? nodes : -1;
+    }
+    __syncthreads();
+    const int nodeCount = sNodes;
+    if (nodeCount < 0) return;
+#pragma unroll
+    for (int t = 0; t < kBuildTiles; t++) {
+        if (t >= tiles) break;
+        const int i = t * kBuildThreads + tid;
+        const float extX = i < n ? system_extent(boxes, key[t], bits) : 0.f;
+        int wlo, whi;
+        warp_levels(lv[t], bits, wlo, whi);
+        write_nodes(i, key[t], extX, lv[t], wlo, whi, off[t * 32 + w], levelOff, bits, maxNodes, nodeCount, nCB, nParent,
+                    nFirst, nMeta);
     }
 }
 
@@ -614,6 +740,16 @@ cudaError_t bh_launch_tree_count(const uint64_t* keys, int n, int bits, uint8_t*
                                  cudaStream_t s) {
     const int blocks = (n + kTreeThreads - 1) / kTreeThreads;
     k_tree_count<<<blocks, kTreeThreads, 0, s>>>(keys, n, bits, delta, blockLevel);
+    return cudaGetLastError();
+}
+
+bool bh_tree_build_one_launch(int n) { return n <= kBuildBodies; }
+
+cudaError_t bh_launch_tree_build_small(const uint64_t* keys, int n, int bits, int maxNodes, const DevBox* box,
+                                       const DevBox* boxes, uint8_t* delta, DevTreeInfo* info, int2* nCB, int* nParent,
+                                       int* nFirst, int* nMeta, int* err, cudaStream_t s) {
+    k_tree_build_small<<<1, kBuildThreads, 0, s>>>(keys, n, bits, maxNodes, box, boxes, delta, info, nCB, nParent, nFirst,
+                                                   nMeta, err);
     return cudaGetLastError();
 }
 
