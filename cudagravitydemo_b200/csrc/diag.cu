@@ -73,7 +73,8 @@ k_diag_moments(const float4* __restrict__ pos, const float3* __restrict__ vel, i
 // half), so that all rows do the same work; block (r, y) takes part y of the
 // row's tiles and writes sum m_i sum_j m_j / r_ij (softened).  FP64 pipe bound
 // as the direct sum is, 13 operations a pair: 65,537 bodies 7.6 -> 2.2 ms, 1M 1180 -> 436,
-// against one ordered pair at a time, one target per thread.
+// against one ordered pair at a time, one target per thread.  A block whose sum is
+// not finite takes it again with rsqrt() (1M with a body at infinity: 588, 1176 before).
 constexpr int kPotThreads = 128;
 constexpr int kRow = 2 * kPotThreads;
 
@@ -109,22 +110,34 @@ k_diag_potential(const float4* __restrict__ pos, int n, int rows, int perPart, d
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
                     const double dx = xy.x - x[k], dy = xy.y - y[k], dz = zm.x - z[k];
-                    const double t = mass_over_r<decltype(edges)::value>(zm.y, fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+                    const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
+                    double t;
+                    if (decltype(edges)::value) {  // half of either body's share: they differ where a mass is 0 or infinite
+                        const double ri = rsqrt(r2);
+                        t = 0.5 * (m[k] * (zm.y * ri) + zm.y * (m[k] * ri));
+                    } else {
+                        t = mass_over_r(zm.y, r2);
+                    }
                     phi[k] += own && base + j <= id[k] ? 0.0 : t;
                 }
             };
             if (d == 0) {
                 for (int j = 0; j < cnt; j++) add(j, true);
+            } else if (decltype(edges)::value) {
+#pragma unroll 1
+                for (int j = 0; j < cnt; j++) add(j, false);
             } else {
 #pragma unroll 4
                 for (int j = 0; j < cnt; j++) add(j, false);
             }
         }
-        return (id[0] < n ? m[0] * phi[0] : 0.0) + (id[1] < n ? m[1] * phi[1] : 0.0);
+        const double f0 = decltype(edges)::value ? phi[0] : m[0] * phi[0], f1 = decltype(edges)::value ? phi[1] : m[1] * phi[1];
+        return (id[0] < n ? f0 : 0.0) + (id[1] < n ? f1 : 0.0);
     };
     double v[1] = {sum(std::false_type())};
-    // a pair at distance 0 or infinity: once more, with these
-    if (__syncthreads_or(!isfinite(v[0]))) v[0] = sum(std::true_type());
+    // a pair at distance 0 or infinity, a mass that is not finite, a softening
+    // whose square is subnormal: once more with rsqrt()
+    if (__syncthreads_or(!isfinite(v[0])) && n > 1) v[0] = sum(std::true_type());
     block_sum<1, kPotThreads>(v);
     if (threadIdx.x == 0) partial[(size_t)blockIdx.y * rows + row] = v[0];
 }

@@ -5,7 +5,12 @@
 // bits, so y^2 is exact and h is rounded once).  1/sqrt(x) = y (1 - h)^(-1/2)
 // and its cube follow from the binomial series, whose first term left out is
 // 5/16 h^3 < 2^-58 and 35/16 h^3 < 2^-55: below the rounding of a double sum's
-// terms, in 5 and 7 operations.
+// terms, in 6 and 7 operations.
+//
+// Both hold for finite m and normal, finite x.  Anything else (a distance of 0
+// or infinity, a softening whose square is subnormal, a mass that is not
+// finite) comes out infinite or NaN, never as a wrong finite number, so a sum
+// that is finite is right and one that is not is taken again with rsqrt().
 #pragma once
 
 __device__ __forceinline__ double rsqrt64_seed(double x) {
@@ -14,7 +19,7 @@ __device__ __forceinline__ double rsqrt64_seed(double x) {
     return y;
 }
 
-// m / x^(3/2), 0 < x < inf
+// m / x^(3/2)
 __device__ __forceinline__ double mass_over_r3(double m, double x) {
     const double y = rsqrt64_seed(x), y2 = y * y;
     const double h = fma(-x, y2, 1.0);
@@ -22,14 +27,10 @@ __device__ __forceinline__ double mass_over_r3(double m, double x) {
     return fma(f, h * fma(1.875, h, 1.5), f);
 }
 
-// m / sqrt(x), 0 < x < inf; with kEdges also x = 0 and x = inf, where h is not a
-// number: a small one in its place lets y = inf and y = 0 come through the series
-// (5% of a pair sum, so the sums ask for it only when they have to).
-template <bool kEdges>
+// m / sqrt(x)
 __device__ __forceinline__ double mass_over_r(double m, double x) {
     const double y = rsqrt64_seed(x);
-    double h = fma(-x, y * y, 1.0);
-    if (kEdges) h = __hiloint2double(__double2hiint(h) & 0x40000000 ? 0x3e000000 : __double2hiint(h), __double2loint(h));
+    const double h = fma(-x, y * y, 1.0);
     const double f = m * y;
     return fma(f, h * fma(0.375, h, 0.5), f);
 }
