@@ -185,6 +185,9 @@ __device__ __forceinline__ void sts_f(unsigned a, float v) { asm volatile("st.sh
 __device__ __forceinline__ void sts_f4(unsigned a, float4 v) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
 }
+// The lanes meet.  Volatile as the accesses above, which name no memory: the
+// compiler keeps all of them in order.
+__device__ __forceinline__ void sync_warp() { asm volatile("bar.warp.sync 0xffffffff;" ::: "memory"); }
 
 // A warp's shared memory, byte offsets from its base:
 //   list   the interaction list as four arrays of kListCap floats: x[], y[], z[], m[]
@@ -399,7 +402,7 @@ k_walk(const WalkArgs a) {
         }
 #pragma unroll
         for (unsigned k = 0; k < kSums; k++) sts_f(sl + Mem::sum + 128u * k, 0.f);  // this lane's column only
-        __syncwarp();
+        sync_warp();
 
         // interactions with list entries [0, cnt); partial sums Kahan-added
         auto kahan = [&](float ax, float ay, float az, unsigned S) {
@@ -665,7 +668,7 @@ k_walk(const WalkArgs a) {
                 top += pushed;
                 maxTop = top > maxTop ? top : maxTop;
             }
-            __syncwarp();
+            sync_warp();
             if (listLen > kListCap - 64) {
                 // the whole blocks of 32 entries; what is left moves to the front
                 const int whole = listLen & ~31;
@@ -677,12 +680,13 @@ k_walk(const WalkArgs a) {
                 const unsigned L = left ? sl + 4u * whole : sm;
                 const float4 e = make_float4(lds_f(L), lds_f(L + Mem::listArray), lds_f(L + 2 * Mem::listArray),
                                              lds_f(L + 3 * Mem::listArray));
-                __syncwarp();
+                sync_warp();
                 append(e, left, lane);
-                __syncwarp();
+                sync_warp();
             }
         }
         if (overflow && lane == 0) bh_set_error(err, BH_ERR_STACK_OVERFLOW);
+        sync_warp();  // (an overflow left its round after other lanes' entries were appended)
         if (listLen > 0) {
             // the last block, filled up with massless copies of its last entry
             // (they add zero wherever that entry's own term is finite)
@@ -690,13 +694,13 @@ k_walk(const WalkArgs a) {
             const unsigned L = sm + 4u * (listLen - 1);
             append(make_float4(lds_f(L), lds_f(L + Mem::listArray), lds_f(L + 2 * Mem::listArray), 0.f),
                    listLen + lane < whole, listLen + lane);
-            __syncwarp();
+            sync_warp();
             flush(whole);
             countInteractions(listLen, nValid);
             if (lane == 0) sts_i(sm + Mem::group + 4, lds_i(sm + Mem::group + 4) + listLen);
         }
         if (a.groupLen && lane == 0) a.groupLen[lds_i(sm + Mem::group)] = lds_i(sm + Mem::group + 4);
-        __syncwarp();
+        sync_warp();
         // results of one body: acceleration, |a|, and the fused kick-drift
         auto finish = [&](int bi, float bx, float by, float bz, float bm_, unsigned S) {
             float gx = lds_f(S), gy = lds_f(S + 128), gz = lds_f(S + 256);
