@@ -490,7 +490,9 @@ class Simulation:
                 "group_votes": st.groupVotes, "status": code}
 
     def profile(self, nsteps: int = 3) -> dict:
-        """Mean ms per stage over nsteps real steps (events between stages)."""
+        """Mean ms per stage over nsteps real steps (events between stages).
+        Up to 2,048 bodies tree_count holds all of tree_count, tree_scan and
+        tree_nodes (one launch)."""
         names = ["keys", "sort", "reorder", "tree_count", "tree_scan", "tree_nodes", "tree_mass", "criterion", "walk"]
         ms = (C.c_float * len(names))()
         _check(lib().bh_sim_profile(self._h, nsteps, ms), "bh_sim_profile")

@@ -64,12 +64,12 @@ cudaError_t bh_launch_tree_scan(int* blockLevel, int nblocks, int n, int bits, i
 cudaError_t bh_launch_tree_nodes(const uint64_t* keys, const uint8_t* delta, int n, int bits,
                                  const int* blockLevel, const DevTreeInfo* info, int maxNodes, const DevBox* boxes,
                                  int2* nCB, int* nParent, int* nFirst, int* nMeta, cudaStream_t s);
-// cooperative launch; bar: one device word for the grid barrier
 // The three above in one launch, for n bodies that one block can take.
 bool bh_tree_build_one_launch(int n);
 cudaError_t bh_launch_tree_build_small(const uint64_t* keys, int n, int bits, int maxNodes, const DevBox* box,
                                        const DevBox* boxes, uint8_t* delta, DevTreeInfo* info, int2* nCB, int* nParent,
                                        int* nFirst, int* nMeta, int* err, cudaStream_t s);
+// cooperative launch (one block for few bodies); bar: one device word for the grid barrier
 cudaError_t bh_launch_tree_mass(const float4* pos, const uint8_t* delta, int n, int bits, const DevTreeInfo* info,
                                 const int2* nCB, float4* nCom, WalkNode* wn, const int* nFirst, int* nCount,
                                 unsigned* bar, int* err, cudaStream_t s);

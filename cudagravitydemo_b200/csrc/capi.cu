@@ -7,10 +7,13 @@
 // kernels with no host synchronisation inside:
 //   k_bbox (world box on the device, histograms zeroed)
 //   k_morton (keys + radix digit histograms)
-//   k_sort_pass x ceil(3*bits/8), or k_sort_cluster for small n
+//   k_sort_pass x ceil(3*bits/8)
 //   k_reorder (pos, vel, body ids)
 //   k_tree_count, k_tree_scan, k_tree_nodes, k_tree_mass [, k_tree_export]
 //   k_walk (+ fused kick-drift)
+// Few bodies: k_box_keys_small for the first two (one system of up to 8,192),
+// k_sort_cluster for the passes (up to 32,768), k_tree_build_small for count, scan
+// and nodes (up to 2,048), k_tree_mass_small for k_tree_mass (up to 4,096).
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>

@@ -92,7 +92,7 @@ constexpr int kMinBlocksWide = BH_WALK_MIN_BLOCKS_WIDE;
 // Few 32-body groups: the time is one long group's chain of rounds, and warps in
 // other slots hide nothing.  More registers (3 blocks, up to 168; 138 to 150 used)
 // let one warp overlap its own entries: a list of 224 takes 3,650 cycles instead
-// of 7,550 (the FMA pipe alone needs 3,600), a vote unrolled whole 1,120 instead of
+// of 7,550 (the dispatch port alone needs 3,600), a vote unrolled whole 1,120 instead of
 // 1,500.  Walk before and after, us, theta 0.5 Plummer spheres unless said: 1,000
 // bodies 42 and 39, 4,000 76 and 66, 16,384 92 and 80, 36,000 145 and 133, 60,000
 // 170 and 164, 100,000 203 and 195; disks of 80,000 171 and 145, learned of 100,000
@@ -864,14 +864,19 @@ static cudaError_t launch_walk_variant(Kernel kernel, const WalkArgs& a, int max
     // How many warps share the groups.  A walk of few groups launches no warps
     // that would only find the cursor at its end, and its blocks spread over the
     // SMs (512 groups taken by the first warps of a full grid sat on few SMs: 155
-    // us at 16,384 bodies, 93 with a grid of their own).  Up to ten groups per
-    // sub-partition, half of them plus one are walked at once: the groups come
-    // longest first, so a warp that is done takes a short one, and fewer at once
-    // leave no half-empty last wave (walk of theta 0.5 disks / Plummer spheres, us
-    // with six warps per sub-partition and with this many, all in 80 registers:
-    // 60,000 bodies 146 / 168 and 143 / 167, 80,000 180 / 199 and 165 / 180, 100,000
-    // 206 / 211 and 173 / 195, 150,000 235 / 250 and 220 / 244; half of them without
-    // the one more: 134 / 200 at 60,000, Plummer spheres have a few long groups).
+    // us at 16,384 bodies, 93 with a grid of their own).  Where half of a
+    // sub-partition's groups plus one is fewer than the warps that it could hold,
+    // that many are walked at once: the groups come longest first, so a warp that
+    // is done takes a short one, and fewer at once leave no half-empty last wave.
+    // That is so at six to eight groups per sub-partition in the build for many
+    // groups and at four in the 64-body one, both 113,665 to 151,552 bodies; below,
+    // the few-groups build holds no more than three and takes them all.  Walk of
+    // theta 0.5 disks / Plummer spheres, us, all warps and this many: 114,000 bodies
+    // 239 / 241 and 211 / 215, 128,000 246 / 246 and 221 / 230, 144,000 250 / 254 and
+    // 224 / 248; learned 306 / 458 and 298 / 469, 321 / 518 and 303 / 496, 334 / 524 and
+    // 321 / 474; 64-body groups at 128,000 336 / 325 and 280 / 275.  Without an order
+    // (accelerations of a state, the drop-in walk) build and walk together are the
+    // same within 2%.
     const int perGroup = wide ? 64 : 32, sms = bh_sm_count();
     const long long groups = a.groupTable ? a.groups : (a.n + perGroup - 1) / perGroup;
     const long long half = (groups - 1) / (2ll * kWarpsPerBlock * sms) + 1;  // rounded up

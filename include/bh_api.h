@@ -166,7 +166,8 @@ int bh_sim_accel_magnitudes(bh_sim* sim, float* aMag, int toHost);
  * so the stages run back to back as in a graph replay); msOut[9] = mean milliseconds of: keys (box + Morton), sort,
  * reorder, tree count, tree scan, tree nodes, tree mass (+ reference-layout
  * export when enabled), learned criterion (group features + budget selection;
- * about 0 in the other modes), walk + kick-drift. */
+ * about 0 in the other modes), walk + kick-drift.  Up to 2,048 bodies count, scan
+ * and nodes are one launch, all of it in tree count; the other two read about 0. */
 int bh_sim_profile(bh_sim* sim, int nsteps, float* msOut);
 /* Kernel launches one step issues. */
 int bh_sim_kernels_per_step(const bh_sim* sim);
